@@ -222,18 +222,12 @@ int ensure_c4_apexes(jgpm_graph* g) {
   JGPM_CUDA_TRY(cudaMemcpyAsync(h, dctr, sizeof(h), cudaMemcpyDeviceToHost, s));
   JGPM_CUDA_TRY(cudaStreamSynchronize(s));
   const int64_t nsmall = (int64_t)h[0], nlarge = (int64_t)h[1], nmid = (int64_t)h[2];
-  int32_t *ds = nullptr, *dm = nullptr, *dl = nullptr;
-  int arc = gmalloc((void**)&ds, std::max<int64_t>(1, nsmall) * 4, s);
-  if (!arc) arc = gmalloc((void**)&dm, std::max<int64_t>(1, nmid) * 4, s);
-  if (!arc) arc = gmalloc((void**)&dl, std::max<int64_t>(1, 2 * nlarge) * 4, s);
-  if (arc) {
-    gfree(ds, s);
-    gfree(dm, s);
-    return arc;
-  }
-  g->d_c4_small = ds;
-  g->d_c4_mid = dm;
-  g->d_c4_large = dl;
+  // the graph gets the lists when they are complete
+  PoolBuf bs{s}, bm{s}, bl{s};
+  if ((rc = bs.alloc((size_t)nsmall * 4)) || (rc = bm.alloc((size_t)nmid * 4)) ||
+      (rc = bl.alloc((size_t)nlarge * 8)))
+    return rc;
+  int32_t *ds = (int32_t*)bs.p, *dm = (int32_t*)bm.p, *dl = (int32_t*)bl.p;
   if (nsmall)
     JGPM_CUDA_TRY(cudaMemcpyAsync(ds, small.p, nsmall * 4, cudaMemcpyDeviceToDevice, s));
   if (nmid)
@@ -258,6 +252,10 @@ int ensure_c4_apexes(jgpm_graph* g) {
     JGPM_CUDA_TRY(cudaMemcpyAsync(g->c4_large_keys.data(), lkey2.p, (size_t)nlarge * 8,
                                   cudaMemcpyDeviceToHost, s));
   JGPM_CUDA_TRY(cudaStreamSynchronize(s));
+  g->d_c4_small = ds;
+  g->d_c4_mid = dm;
+  g->d_c4_large = dl;
+  bs.p = bm.p = bl.p = nullptr;
   g->c4_nsmall = nsmall;
   g->c4_nmid = nmid;
   g->c4_nlarge = nlarge;

@@ -8,6 +8,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <cstdio>
@@ -430,7 +431,16 @@ int grid_for(int64_t work, int threads = 256) {
 
 }  // namespace
 
+namespace {
+std::atomic<int64_t> g_fail_alloc{-1};  // jgpm_fail_alloc_
+}
+
 int gmalloc(void** p, size_t bytes, cudaStream_t s) {
+  if (g_fail_alloc.load(std::memory_order_relaxed) >= 0 && g_fail_alloc.fetch_sub(1) == 0) {
+    *p = nullptr;
+    jgpm_set_error_("device allocation refused (jgpm_fail_alloc_)");
+    return JGPM_ENOMEM;
+  }
   int dev = 0;
   cudaGetDevice(&dev);
   cudaMemPool_t pool = device_pool(dev);
@@ -469,6 +479,12 @@ struct DevBuf {
   explicit DevBuf(cudaStream_t stream) : s(stream) {}
   ~DevBuf() {
     if (p) gfree(p, s);
+  }
+  // Hands the buffer over to a graph.
+  template <typename T>
+  void publish(T** to) {
+    *to = (T*)p;
+    p = nullptr;
   }
 };
 
@@ -706,7 +722,10 @@ int ensure_dag(jgpm_graph* g) {
   const int64_t m = g->m;
   const int32_t n = g->n;
   int rc;
-  if ((rc = dalloc(&g->d_dag_rowptr, (size_t)n + 1, g->stream))) return rc;
+  // the graph gets the arrays when they are complete: a call that failed half-way is as if it
+  // had not been made
+  DevBuf rowptr(s), col(s);
+  if ((rc = dalloc((int64_t**)&rowptr.p, (size_t)n + 1, s))) return rc;
   // one bit per arc, and one prefix per 32 arcs: nothing of the arcs' size but the arcs is
   // written (33 M arcs: 0.80 ms with a source, a flag and a position for each arc)
   const int64_t words = (m + 31) >> 5;
@@ -738,19 +757,21 @@ int ensure_dag(jgpm_graph* g) {
                                                cub::Sum(), (int64_t)0, words + 1, s));
   // every edge is one DAG arc
   const int64_t total = m / 2;
-  if ((rc = dalloc(&g->d_dag_col, total, s))) return rc;
+  if ((rc = dalloc((int32_t**)&col.p, total, s))) return rc;
   if (words > 0)
     k_orient_scatter<<<grid_for(m), 256, 0, s>>>(g->d_col, keep, (int64_t*)pos.p, m,
-                                                 g->d_dag_col);
+                                                 (int32_t*)col.p);
   k_dag_rowptr<<<grid_for((int64_t)n + 1), 256, 0, s>>>(g->d_rowptr, keep,
                                                         (int64_t*)pos.p, n, m, total,
-                                                        g->d_dag_rowptr, (int*)st.p);
+                                                        (int64_t*)rowptr.p, (int*)st.p);
   JGPM_CUDA_TRY(cudaGetLastError());
-  g->m_dag = total;
   int h = 0;
   JGPM_CUDA_TRY(cudaMemcpyAsync(&h, st.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   JGPM_CUDA_TRY(cudaStreamSynchronize(s));
+  g->m_dag = total;
   g->max_out_degree = h;
+  rowptr.publish(&g->d_dag_rowptr);
+  col.publish(&g->d_dag_col);
   return JGPM_OK;
 }
 
@@ -1169,17 +1190,14 @@ uint64_t rank_dag_bytes(const jgpm_graph* g) {
 int ensure_control(jgpm_graph* g) {
   if (g->d_ctl) return JGPM_OK;
   int rc;
-  if (!g->ev0) {
-    JGPM_CUDA_TRY(cudaEventCreate(&g->ev0));
-    JGPM_CUDA_TRY(cudaEventCreate(&g->ev1));
-  }
-  if ((rc = dalloc(&g->d_ctl, 1, g->stream))) return rc;
-  g->h_ctl = ctl_slot();
-  if (!g->h_ctl) {
+  if (!g->ev0) JGPM_CUDA_TRY(cudaEventCreate(&g->ev0));
+  if (!g->ev1) JGPM_CUDA_TRY(cudaEventCreate(&g->ev1));
+  if (!g->h_ctl && !(g->h_ctl = ctl_slot())) {
     jgpm_set_error_("pinned host allocation of a control block failed");
     return JGPM_ENOMEM;
   }
   memset(g->h_ctl, 0, sizeof(DevControl));
+  if ((rc = dalloc(&g->d_ctl, 1, g->stream))) return rc;
   return JGPM_OK;
 }
 
@@ -1205,21 +1223,36 @@ int ensure_aux(jgpm_graph* g, size_t bytes) {
   return JGPM_OK;
 }
 
-void free_graph_device(jgpm_graph* g) {
-  gfree(g->d_rowptr, g->stream);
-  gfree(g->d_col, g->stream);
-  gfree(g->d_dag_rowptr, g->stream);
-  gfree(g->d_dag_col, g->stream);
-  gfree(g->d_keep, g->stream);
-  gfree(g->d_rank_rowptr, g->stream);
-  gfree(g->d_rank_col, g->stream);
-  gfree(g->d_c4_small, g->stream);
-  gfree(g->d_c4_mid, g->stream);
-  gfree(g->d_c4_large, g->stream);
+namespace {
+// Gives back every array of a graph but its control block; the graph is as before its upload.
+void drop_arrays(jgpm_graph* g) {
+  auto drop = [&](auto*& p) {
+    gfree(p, g->stream);
+    p = nullptr;
+  };
+  drop(g->d_rowptr);
+  drop(g->d_col);
+  drop(g->d_dag_rowptr);
+  drop(g->d_dag_col);
+  drop(g->d_keep);
+  drop(g->d_rank_rowptr);
+  drop(g->d_rank_col);
+  drop(g->d_c4_small);
+  drop(g->d_c4_mid);
+  drop(g->d_c4_large);
+  drop(g->d_scratch);
+  drop(g->d_aux);
   free_rank_dag(g);
+  g->aux_bytes = g->scratch_bytes = 0;
+  g->c4_nsmall = -1;
+  g->c4_nmid = g->c4_nlarge = g->c4_ndense = 0;
+  g->c4_large_keys.clear();
+}
+}  // namespace
+
+void free_graph_device(jgpm_graph* g) {
+  drop_arrays(g);
   gfree(g->d_ctl, g->stream);
-  gfree(g->d_scratch, g->stream);
-  gfree(g->d_aux, g->stream);
   ctl_release(g->h_ctl);
   if (g->ev0) cudaEventDestroy(g->ev0);
   if (g->ev1) cudaEventDestroy(g->ev1);
@@ -1389,50 +1422,20 @@ int evict_graph(jgpm_graph* g, std::vector<int64_t>& h_rowptr, std::vector<int32
                                     cudaMemcpyDeviceToHost, g->stream));
   }
   JGPM_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  gfree(g->d_rowptr, g->stream);
-  gfree(g->d_col, g->stream);
-  gfree(g->d_dag_rowptr, g->stream);
-  gfree(g->d_dag_col, g->stream);
-  gfree(g->d_keep, g->stream);
-  gfree(g->d_rank_rowptr, g->stream);
-  gfree(g->d_rank_col, g->stream);
-  gfree(g->d_c4_small, g->stream);
-  gfree(g->d_c4_mid, g->stream);
-  gfree(g->d_c4_large, g->stream);
-  free_rank_dag(g);
-  gfree(g->d_scratch, g->stream);
-  gfree(g->d_aux, g->stream);
-  g->d_aux = nullptr;
-  g->aux_bytes = 0;
-  g->d_rank_rowptr = nullptr;
-  g->d_rank_col = nullptr;
-  g->d_c4_small = nullptr;
-  g->d_c4_mid = nullptr;
-  g->d_c4_large = nullptr;
-  g->c4_nsmall = -1;
-  g->c4_nmid = 0;
-  g->c4_nlarge = 0;
-  g->c4_ndense = 0;
-  g->c4_large_keys.clear();
-  g->d_rowptr = nullptr;
-  g->d_col = nullptr;
-  g->d_dag_rowptr = nullptr;
-  g->d_dag_col = nullptr;
-  g->d_keep = nullptr;
-  g->d_scratch = nullptr;
-  g->scratch_bytes = 0;
+  drop_arrays(g);
   return JGPM_OK;
 }
 
-// Uploads an evicted graph again and rebuilds its DAG and root tiers.
+// Uploads an evicted graph again and rebuilds its DAG and root tiers.  On an error the graph stays
+// evicted.
 int restore_graph(jgpm_graph* g, const std::vector<int64_t>& h_rowptr,
                   const std::vector<int32_t>& h_col) {
   if (g->d_rowptr) return JGPM_OK;
-  int rc;
-  if ((rc = upload_csr(g, h_rowptr.data(), h_col.data(), g->n, (int64_t)h_col.size(), 0, 0)))
-    return rc;
-  if ((rc = ensure_dag(g))) return rc;
-  return ensure_tiers(g);
+  int rc = upload_csr(g, h_rowptr.data(), h_col.data(), g->n, (int64_t)h_col.size(), 0, 0);
+  if (!rc) rc = ensure_dag(g);
+  if (!rc) rc = ensure_tiers(g);
+  if (rc) drop_arrays(g);
+  return rc;
 }
 
 // Device bytes held by a resident graph's arrays.
@@ -1447,3 +1450,7 @@ uint64_t graph_device_bytes(const jgpm_graph* g) {
 }
 
 }  // namespace jgpm
+
+// Test hook: the `after`-th allocation from the pools from now on (0 = the next), by any thread,
+// fails with JGPM_ENOMEM; a negative number calls it off.
+extern "C" void jgpm_fail_alloc_(int64_t after) { jgpm::g_fail_alloc.store(after); }

@@ -206,7 +206,10 @@ int launch_batch(jgpm_server* s, Slot& slot) {
     if (!pg.resident) {
       int rc = make_resident(s, q->graph_id, with_q);
       if (rc == JGPM_EBUSY) continue;
-      if (rc) return rc;
+      if (rc) {  // nothing is launched: every query stays pending
+        for (auto& b : batch) s->graphs[b->graph_id].inflight--;
+        return rc;
+      }
     }
     if (over_budget(s, with_q) && (!batch.empty() || s->inflight_frontier > 0))
       continue;  // wait for in-flight work to release memory
