@@ -280,6 +280,7 @@ struct Offsets {
   int64_t a_end = 0, b_end = 0, out_end = 0;  // totals, where staging needs them
   OffsetCheck* check = nullptr;
   cudaStream_t stream = nullptr;
+  bool checked = false;  // on the host, or the device check's result is read
   bool a_null = false, b_null = false;  // operand or output arrays that only empty lists allow
   // Returns JGPM_OK or the error.  need_totals: host arrays have to be sized.
   int init(const char* who, const int64_t* a_off, const int64_t* b_off, const int64_t* out_off,
@@ -305,6 +306,7 @@ struct Offsets {
     JGPM_CUDA_TRY(out.init(out_off, (size_t)nops + 1, s));
     if (gmalloc((void**)&check, sizeof(OffsetCheck), s)) return JGPM_ENOMEM;
     JGPM_CUDA_TRY(cudaMemsetAsync(check, 0xff, sizeof(OffsetCheck), s));
+    checked = host;
     if (host) return JGPM_OK;
     k_check_offsets<<<(int)std::min<int64_t>((nops + 255) / 256, 148 * 8), 256, 0, s>>>(
         a.d, b.d, out.d, op, nops, check);
@@ -319,8 +321,10 @@ struct Offsets {
     return verdict(who);
   }
   bool missing() const { return (a_end > 0 && a_null) || (b_end > 0 && b_null); }
-  // The device check's result (the stream is idle after it).
+  // The device check's result, if it is not read yet (the stream is idle then).
   int verdict(const char* who) {
+    if (checked) return JGPM_OK;
+    checked = true;
     OffsetCheck h;
     JGPM_CUDA_TRY(cudaMemcpyAsync(&h, check, sizeof(h), cudaMemcpyDeviceToHost, stream));
     JGPM_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -441,15 +445,18 @@ int jgpm_setop_batch(int op, const int32_t* a, const int64_t* a_off, const int32
       op, da.d, off.a.d, db.d, off.b.d, nops, dup.d, dex.d, dcounts, mat ? dout : nullptr,
       mat ? off.out.d : nullptr, off.check);
   cudaError_t e = cudaGetLastError();
+  // a refused call writes nothing: the staged results are copied back once the verdict is read
+  if (e == cudaSuccess && (rc = off.verdict("jgpm_setop_batch"))) return rc;
   if (e == cudaSuccess && counts_host)
     e = cudaMemcpyAsync(counts, dcounts, nops * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && out_host && off.out_end > 0)
     e = cudaMemcpyAsync(out, dout, off.out_end * 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     jgpm_set_error_(std::string("jgpm_setop_batch: ") + cudaGetErrorString(e));
     return JGPM_ECUDA;
   }
-  return off.verdict("jgpm_setop_batch");
+  return JGPM_OK;
 }
 
 int jgpm_setop_split_batch(int kind, const int32_t* a, const int64_t* a_off, const int32_t* b,
@@ -496,6 +503,7 @@ int jgpm_setop_split_batch(int kind, const int32_t* a, const int64_t* a_off, con
   if (err == cudaSuccess) err = oc.back(s);
   if (err == cudaSuccess) err = od.back(s);
   if (err == cudaSuccess) err = oe.back(s);
+  if (err == cudaSuccess && off.checked) err = cudaStreamSynchronize(s);
   if (err != cudaSuccess) {
     jgpm_set_error_(std::string("jgpm_setop_split_batch: ") + cudaGetErrorString(err));
     return JGPM_ECUDA;

@@ -56,10 +56,14 @@ def test_results_at_step_edges(gpu, op):
             assert (got[oo[i] + len(x): oo[i + 1]] == -7).all(), i
 
 
+# counts on the host with everything else on the device: they are staged, and a refused call
+# must not copy the staging buffer back
+@pytest.mark.parametrize("counts_at", ["cuda", "host"])
 @pytest.mark.parametrize("where", ["host", "cuda"])
-def test_offset_errors(gpu, where):
+def test_offset_errors(gpu, where, counts_at):
     a = torch.arange(8, dtype=torch.int32, device="cuda")
-    counts = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+    counts = torch.full((2,), -1, dtype=torch.int32,
+                        device="cuda" if counts_at == "cuda" else "cpu")
     out = torch.zeros(8, dtype=torch.int32, device="cuda")
 
     def off(*x):
@@ -78,3 +82,30 @@ def test_offset_errors(gpu, where):
         if code:
             assert counts.cpu().tolist() == [-1, -1]
     assert counts.cpu().tolist() == [4, 4]
+
+
+@pytest.mark.parametrize("counts_at", ["cuda", "host"])
+@pytest.mark.parametrize("where", ["host", "cuda"])
+def test_refused_split_writes_nothing(gpu, where, counts_at):
+    a = torch.arange(8, dtype=torch.int32, device="cuda")
+    c, d = torch.full_like(a, -7), torch.full_like(a, -7)
+    counts = torch.full((4,), -1, dtype=torch.int32,
+                        device="cuda" if counts_at == "cuda" else "cpu")
+    i64 = ctypes.c_int64
+
+    def off(*x):
+        t = torch.tensor(x, dtype=torch.int64)
+        return t.cuda() if where == "cuda" else t
+
+    def split(ao, bo):
+        return gpu.lib().jgpm_setop_split_batch(
+            gpu.SPLIT_DIF_INT, _p(a), _p(ao, i64), _p(a), _p(bo, i64), 2, None, _p(counts),
+            _p(c), _p(d), None)
+
+    good = off(0, 4, 8)
+    torch.cuda.synchronize()
+    for ao, bo in [(off(0, 5, 3), good), (good, off(4, 2, 8)), (off(-1, 4, 8), good)]:
+        assert split(ao, bo) == -1
+        assert counts.tolist() == [-1] * 4 and (c == -7).all() and (d == -7).all()
+    assert split(good, good) == 0
+    assert counts.tolist()[0] in (0, 4)
