@@ -33,7 +33,8 @@ __global__ void k_c4_classify(const eid_t* rp, const vid_t* col, vid_t n, vid_t*
   // an apex has two lower-ranked neighbours, so none lies below vmin either
   const vid_t vmin = c4_first_id(rp, n);
   if (first == 0 && lane == 0) counters[4] = (unsigned long long)vmin;
-  for (int64_t v = vmin + first; v < n; v += warps) {
+  // from the top: the lists come out roughly heaviest first, as the kernels that drain them want
+  for (int64_t v = (int64_t)n - 1 - first; v >= vmin; v -= warps) {
     const eid_t b = rp[v];
     const int d = (int)(rp[v + 1] - b);
     int cut = 0;
