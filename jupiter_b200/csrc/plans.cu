@@ -25,6 +25,8 @@
 //                 induced/non-induced identities of 4-vertex graphlets.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -98,6 +100,7 @@ struct PlanArgs {
   int32_t* scratch;
   int64_t cap;  // entries per scratch list (4 lists per warp)
   int2* heavy;  // queue of the arcs that are split (null: none is)
+  int64_t heavy_cap;  // arcs it takes; those past it run unsplit
 };
 
 struct Lists {
@@ -120,19 +123,16 @@ __device__ __forceinline__ bool has(const int32_t* list, int n, int32_t key) {
   return p < n && ld32<RO>(list + p) == key;
 }
 
-// |A & B|, A of either kind, B a graph row: the keys of the shorter list are looked up in the
-// longer one (warp-uniform result).
-template <bool ARO>
+// |A & B| of two lists, either of which this warp may have written (plain loads): the keys of the
+// shorter one are looked up in the longer one (warp-uniform result).
 __device__ __forceinline__ int warp_common(const int32_t* a, int na, const int32_t* b, int nb) {
-  const int lane = threadIdx.x & 31;
-  int c = 0;
-  if (na <= nb) {
-    for (int i = lane; i < na; i += 32)
-      if (contains_g(b, nb, ld32<ARO>(a + i))) ++c;
-  } else {
-    for (int i = lane; i < nb; i += 32)
-      if (has<ARO>(a, na, __ldg(b + i))) ++c;
+  if (na > 32 && na > nb) {
+    const int32_t* t = a; a = b; b = t;
+    const int tn = na; na = nb; nb = tn;
   }
+  int c = 0;
+  for (int i = threadIdx.x & 31; i < na; i += 32)
+    if (has<false>(b, nb, a[i])) ++c;
   return warp_sum_int(c);
 }
 
@@ -224,12 +224,14 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
       const int t0 = lower_bound_t<false>(L.W, t, v1);  // v1 is not in W
       const int32_t* T = L.W + t0;
       const int nt = t - t0;
+      if (nt == 0) return 0;
+#pragma unroll 1
       for (int i3 = split.first; i3 < d0; i3 += split.step) {
         const vid_t v3 = __ldg(N0 + i3);
         if (v3 == v1) continue;
         const int32_t* N3 = nbr(a, v3);
         const int d3 = dg(a, v3);
-        const int c = warp_common<false>(T, nt, N3, d3);
+        const int c = warp_common(T, nt, N3, d3);
         if (lane == 0)
           lc += (acc_t)(nt - (has<false>(T, nt, v3) ? 1 : 0)) *
                     (acc_t)(d3 - 1 - (contains_g(N3, d3, v1) ? 1 : 0)) -
@@ -237,28 +239,32 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
       }
     } else if (P == kP4) {
       // v2 in W, v2 != v3: |X|, X = N0 & N3, less v1 (always in X) and v2 where it is in N3
+      if (t == 0 && !STATS) return 0;
+#pragma unroll 1
       for (int i3 = split.first; i3 < d1; i3 += split.step) {
         const vid_t v3 = __ldg(N1 + i3);
         if (v3 == v0) continue;
         const int32_t* N3 = nbr(a, v3);
         const int d3 = dg(a, v3);
         if (STATS && lane == 0) el += (acc_t)d0 + d3;
-        const int tx = warp_intersect_count(N0, d0, N3, d3);
-        const int c = warp_common<false>(L.W, t, N3, d3);
+        const int tx = warp_common(N0, d0, N3, d3);
+        const int c = warp_common(L.W, t, N3, d3);
         if (lane == 0)
           lc += (acc_t)(t - (has<false>(L.W, t, v3) ? 1 : 0)) * (acc_t)(tx - 1) - (acc_t)c;
       }
     } else if (P == kP5) {
       // v4 in W, v4 != v2: |X|, X = W & N2 below v2, less v4 where it is in X
+#pragma unroll 1
       for (int i = split.first; i < t; i += split.step) {
         const vid_t v2 = L.W[i];
         const int32_t* N2 = nbr(a, v2);
         const int d2 = dg(a, v2);
         if (STATS && lane == 0)
           el += (acc_t)prefix_len<false>(L.W, t, v2) + prefix_len<true>(N2, d2, v2);
-        u += (acc_t)warp_common<false>(L.W, i, N2, d2) * (acc_t)(t - 2);  // W[i] = v2: W below it
+        u += (acc_t)warp_common(L.W, i, N2, d2) * (acc_t)(t - 2);  // W[i] = v2: W below it
       }
     } else if (P == kP6) {
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         const int32_t* N2 = nbr(a, v2);
@@ -273,6 +279,7 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
       }
     } else if (P == kP7) {
       // v4 in X = N0 & N2, v4 != v1 (always in X): |W| less v2 and v4 where it is in W
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         if (v2 <= v1) continue;
@@ -280,9 +287,10 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
         const int d2 = dg(a, v2);
         if (STATS && lane == 0) el += (acc_t)d0 + d2;
         const int tx = warp_intersect_count(N0, d0, N2, d2);
-        u += (acc_t)(tx - 1) * (acc_t)(t - 1) - (acc_t)warp_common<false>(L.W, t, N2, d2);
+        u += (acc_t)(tx - 1) * (acc_t)(t - 1) - (acc_t)warp_common(L.W, t, N2, d2);
       }
     } else if (P == kP8) {
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         if (v2 >= v1) continue;
@@ -302,18 +310,20 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
         __syncwarp();
       }
     } else if (P == kP9) {
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         if (v2 <= v1) continue;
         const int32_t* N2 = nbr(a, v2);
         const int d2 = dg(a, v2);
         if (STATS && lane == 0) el += (acc_t)t + d2;
-        const acc_t tx = (acc_t)warp_common<false>(L.W, t, N2, d2);
+        const acc_t tx = (acc_t)warp_common(L.W, t, N2, d2);
         u += tx * (tx - (tx > 0 ? 1 : 0)) / 2;
       }
     } else if (P == kP10) {
       // v4 in W, v4 not v2 or v3: |Y|, Y = N0 & N3, less v2 (always in Y), v1 and v4 where they
       // are in N3; v3 is in W, and v1 in Y, when v1 ~ v3
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         const int32_t* N2 = nbr(a, v2);
@@ -327,7 +337,7 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
           const int d3 = dg(a, v3);
           if (STATS && lane == 0) el += (acc_t)d0 + d3;
           const int ty = warp_intersect_count(N0, d0, N3, d3);
-          const int c = warp_common<false>(L.W, t, N3, d3);
+          const int c = warp_common(L.W, t, N3, d3);
           if (lane == 0) {
             const int b = contains_g(N3, d3, v1) ? 1 : 0;
             lc += (acc_t)(t - 1 - b) * (acc_t)(ty - 1 - b) - (acc_t)(c - 1);
@@ -339,6 +349,7 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
       // v3 in W, v4 in X = N0 & N2, all distinct: |Z|, Z = N1 & N2, less v0 (always in Z), v3
       // where it is in N2 and v4 where it is in N1.  With q = |W & N2|: q of the v3 lie in N2 (and
       // so in X and Z), and q of X lie in N1
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         if (v2 <= v1) continue;
@@ -347,23 +358,26 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
         if (STATS && lane == 0) el += (acc_t)d0 + d2 + d1 + d2;
         const acc_t tx = (acc_t)warp_intersect_count(N0, d0, N2, d2);
         const acc_t tz = (acc_t)warp_intersect_count(N1, d1, N2, d2);
-        const acc_t q = (acc_t)warp_common<false>(L.W, t, N2, d2);
+        const acc_t q = (acc_t)warp_common(L.W, t, N2, d2);
         u += q * ((tx - 2) * (tz - 2) - (q - 1)) +
              ((acc_t)t - 1 - q) * ((tx - 1) * (tz - 1) - q);
       }
     } else if (P == kP12) {
       // v3 < v4 in X = W & N2: |W| less v2, v3 and v4
+#pragma unroll 1
       for (int i2 = split.first; i2 < t; i2 += split.step) {
         const vid_t v2 = L.W[i2];
         const int32_t* N2 = nbr(a, v2);
         const int d2 = dg(a, v2);
         if (STATS && lane == 0) el += (acc_t)t + d2;
-        const acc_t tx = (acc_t)warp_common<false>(L.W, t, N2, d2);
+        const acc_t tx = (acc_t)warp_common(L.W, t, N2, d2);
         if (tx > 1) u += tx * (tx - 1) / 2 * (acc_t)(t - 3);
       }
     } else if (P == kVsgm) {
       // v5 in Z = N1 & N2, v5 != v0 (always in Z); v3 < w in W without v2 and v5, where they are
       // in it: v2 is when v1 ~ v2, and |W & N2| of the v5 are
+      if (t < 2 && !STATS) return 0;
+#pragma unroll 1
       for (int i2 = split.first; i2 < d0; i2 += split.step) {
         const vid_t v2 = __ldg(N0 + i2);
         if (v2 == v1) continue;
@@ -371,7 +385,7 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
         const int d2 = dg(a, v2);
         if (STATS && lane == 0) el += (acc_t)d1 + d2;
         const acc_t tz = (acc_t)warp_intersect_count(N1, d1, N2, d2);
-        const acc_t q = (acc_t)warp_common<false>(L.W, t, N2, d2);
+        const acc_t q = (acc_t)warp_common(L.W, t, N2, d2);
         if (lane == 0) {
           const int64_t m = t - (contains_g(N1, d1, v2) ? 1 : 0);
           lc += q * (acc_t)((m - 1) * (m - 2) / 2) + (tz - 1 - q) * (acc_t)(m * (m - 1) / 2);
@@ -458,13 +472,21 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
 // rows from which it pays: a hub's arc runs hundreds of list operations for each of hundreds of
 // candidates, on one warp for milliseconds after all others have finished.  Such arcs go to a
 // queue that k_plan_heavy drains in kHeavyParts parts each; its candidate lists are built again by
-// every part, a small share of its work.
+// every part, a small share of its work.  R-MAT, P9 in ms, unsplit | rows of 96 | 192 | 384 | 768 on:
+// 8,192 vertices, edge factor 16, a = 0.45, b = 0.2391: 4.16 | 0.80 | 0.82 | 1.29 | 2.19; 30,000
+// vertices, edge factor 8, a = 0.57: 14.7 | 2.3 | 2.5 | 2.8 | 6.6; 131,072 vertices, edge factor 4,
+// a = 0.51: 0.32 | 0.37 | 0.34 | 0.34 | 0.32.  In 8, 16 and 32 parts (192): 0.85, 0.82, 0.89 | 2.2,
+// 2.5, 3.4 | 0.36, 0.34, 0.34; P3, P5, P7, P10 and P12 alike.
 constexpr bool kSplitPlan(int p) { return p >= kP3 && p <= kVsgm; }
 constexpr int kHeavyRow = 192;
 constexpr int kHeavyParts = 16;
-constexpr int64_t kHeavyQueue = (int64_t)1 << 20;  // arcs; those past it run unsplit
+constexpr int64_t kHeavyQueue = (int64_t)1 << 20;  // arcs
+std::atomic<int64_t> g_heavy_cap{kHeavyQueue};     // jgpm_heavy_queue_
 
-template <int P, bool STATS>
+// QUEUE: arcs of two long rows go to a.heavy.  Graphs that can have none run the kernel that does not
+// look for them (P9 of 131,072 vertices, edge factor 4, a = 0.45: 0.30 ms with the test, 0.28 ms
+// without).
+template <int P, bool STATS, bool QUEUE>
 __global__ void __launch_bounds__(256) k_plan(PlanArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t gwarp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -500,11 +522,11 @@ __global__ void __launch_bounds__(256) k_plan(PlanArgs a) {
         v0 = owner(v0, s);
       }
       const vid_t v1 = __ldg(a.col + s);
-      if (kSplitPlan(P) && !STATS && a.heavy && min(dg(a, v0), dg(a, v1)) >= kHeavyRow) {
+      if (QUEUE && min(dg(a, v0), dg(a, v1)) >= kHeavyRow) {
         unsigned long long q = 0;
         if (lane == 0) q = atomicAdd(&a.ctl->counter[1], 1ull);
         q = __shfl_sync(kFull, q, 0);
-        if ((int64_t)q < kHeavyQueue) {
+        if ((int64_t)q < a.heavy_cap) {
           if (lane == 0) a.heavy[q] = make_int2(v0, v1);
           continue;
         }
@@ -532,7 +554,7 @@ __global__ void __launch_bounds__(256) k_plan_heavy(PlanArgs a) {
   L.Y = L.X + a.cap;
   L.Z = L.Y + a.cap;
   acc_t lc = 0, uc = 0, el = 0;
-  const int64_t arcs = min((int64_t)a.ctl->counter[1], kHeavyQueue);
+  const int64_t arcs = min((int64_t)a.ctl->counter[1], a.heavy_cap);
   for (;;) {
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(&a.ctl->counter[2], 1ull);
@@ -641,17 +663,16 @@ int grid_for(int64_t work, int threads = 256) {
 template <int P>
 int launch_plan_t(const PlanArgs& a, bool stats, int grid, cudaStream_t s, int* n) {
   *n = 1;
-  if (stats) {
-    k_plan<P, true><<<grid, 256, 0, s>>>(a);
-    return JGPM_OK;
-  }
-  k_plan<P, false><<<grid, 256, 0, s>>>(a);
   if constexpr (kSplitPlan(P)) {
     if (a.heavy) {
+      k_plan<P, false, true><<<grid, 256, 0, s>>>(a);
       k_plan_heavy<P><<<grid, 256, 0, s>>>(a);
       *n = 2;
+      return JGPM_OK;
     }
   }
+  if (stats) k_plan<P, true, false><<<grid, 256, 0, s>>>(a);
+  else k_plan<P, false, false><<<grid, 256, 0, s>>>(a);
   return JGPM_OK;
 }
 
@@ -724,6 +745,7 @@ int run_literal(jgpm_graph* g, int id, int chunk_size, bool stats, uint64_t* out
   if ((rc = ensure_scratch(g, list_bytes + queue_bytes))) return rc;
   PlanArgs a{};
   a.heavy = queue ? (int2*)((char*)g->d_scratch + list_bytes) : nullptr;
+  a.heavy_cap = std::min<int64_t>(kHeavyQueue, g_heavy_cap.load());
   a.rowptr = dag ? g->d_dag_rowptr : g->d_rowptr;
   a.col = dag ? g->d_dag_col : g->d_col;
   a.n = g->n;
@@ -1181,6 +1203,7 @@ extern "C" int jgpm_count_noalloc(jgpm_graph* g, const char* pattern, int induce
   a.ctl = d.ctl;
   a.scratch = d.scratch;
   a.cap = cap;
+  // no queue: the caller's arrays have no room for one, so hub arcs run on one warp each
   a.slot_begin = 0;
   a.slot_end = dag ? g->m_dag : g->m;
   a.slot_stride = 1;
@@ -1207,3 +1230,6 @@ extern "C" int jgpm_count_noalloc(jgpm_graph* g, const char* pattern, int induce
   *out = cnt;
   return JGPM_OK;
 }
+
+// Test hook: the queue of split arcs takes `arcs` of them (kHeavyQueue at most) from now on.
+extern "C" void jgpm_heavy_queue_(int64_t arcs) { jgpm::g_heavy_cap.store(arcs); }

@@ -128,7 +128,10 @@ __device__ __forceinline__ void contains_u(const int32_t* __restrict__ b, int nb
 
 // Visits the keys of A in order, 32 U at a time while more than 32 are left, else 32: visit(key,
 // valid, in_b) is called by the whole warp for each 32 keys, one per lane.  Four searches at a
-// time are what hides their latency: lists are longer than L1 and mostly cold.
+// time are what hides their latency in the set-op batches, whose lists are long and mostly cold.
+// The plans and list tiers below search one key per lane: their lists are a few ids long on most
+// arcs, and the registers and steps of four searches cost them 5 to 10 % there (P9, P10 and P11 on
+// R-MAT graphs of 131,072 vertices, edge factor 4, a = 0.45).
 template <typename Visit>
 __device__ __forceinline__ void warp_lookup(const int32_t* a, int na, const int32_t* b, int nb,
                                             Visit&& visit) {
@@ -149,10 +152,8 @@ __device__ __forceinline__ void warp_lookup(const int32_t* a, int na, const int3
   }
   if (base < na) {
     const int i = base + lane;
-    int32_t key[1] = {i < na ? __ldg(a + i) : INT32_MAX};
-    bool hit[1];
-    contains_u<1>(b, nb, key, hit);
-    visit(key[0], i < na, hit[0]);
+    const int32_t key = i < na ? __ldg(a + i) : INT32_MAX;
+    visit(key, i < na, i < na && contains_g(b, nb, key));
   }
 }
 
@@ -177,9 +178,10 @@ __device__ __forceinline__ int warp_intersect_count(const int32_t* a, int na, co
     const int d1 = (int)((int64_t)total * (lane + 1) / 32);
     c = merge_segment_count(a, na, b, nb, d0, d1, ex0, ex1);
   } else {
-    warp_lookup(a, na, b, nb, [&](int32_t key, bool valid, bool in_b) {
-      if (valid && in_b && key != ex0 && key != ex1) ++c;
-    });
+    for (int i = lane; i < na; i += 32) {
+      const int32_t key = __ldg(a + i);
+      if (key != ex0 && key != ex1 && contains_g(b, nb, key)) ++c;
+    }
   }
   return warp_sum_int(c);
 }
@@ -196,12 +198,14 @@ __device__ __forceinline__ int warp_intersect(const int32_t* a, int na, const in
     int tn = na; na = nb; nb = tn;
   }
   int written = 0;
-  warp_lookup(a, na, b, nb, [&](int32_t key, bool valid, bool in_b) {
-    const bool f = valid && in_b;
+  for (int base = 0; base < na; base += 32) {
+    const int i = base + lane;
+    const int32_t key = i < na ? __ldg(a + i) : 0;
+    const bool f = i < na && contains_g(b, nb, key);
     const unsigned mask = __ballot_sync(kFull, f);
     if (f) out[written + __popc(mask & ((1u << lane) - 1))] = key;
     written += __popc(mask);
-  });
+  }
   __syncwarp();
   return written;
 }
