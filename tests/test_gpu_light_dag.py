@@ -1,0 +1,63 @@
+"""Graphs whose rows lie outside the adjacency bitmap and are short, so that the lane groups scan
+them: weakly skewed R-MAT graphs, and sparse graphs with planted complete graphs, which bring roots
+of out-degree 32, 33, 63, 64 and 65.  Counts are integers: equality with the oracle, single calls,
+batches and shards."""
+import numpy as np
+import pytest
+
+import oracle_api as O
+
+pytestmark = pytest.mark.gpu
+
+PLAIN = {"triangle": "P0", "4-clique": "P13", "5-clique": "P14", "6-clique": "P15"}
+
+
+def sparse_with_cliques(n, sizes, seed):
+    """A random graph of n vertices and 6 n edges with a complete graph planted for each size."""
+    rng = np.random.default_rng(seed)
+    src, dst = [rng.integers(0, n, 6 * n)], [rng.integers(0, n, 6 * n)]
+    free = rng.permutation(n)
+    for s in sizes:
+        at, free = free[:s], free[s:]
+        i, j = np.triu_indices(s, 1)
+        src.append(at[i])
+        dst.append(at[j])
+    src, dst = np.concatenate(src).astype(np.int32), np.concatenate(dst).astype(np.int32)
+    keep = src != dst
+    return O.build_csr(n, src[keep], dst[keep])
+
+
+def wanted(sym):
+    dag = O.orient(sym)
+    want = {k: O.count(p, dag)[0] for k, p in PLAIN.items()}
+    want["diamond"] = O.count("P2", sym)[0]
+    return want, O.count("induced-tailed-triangle", sym)[0], dag
+
+
+def check(gpu, sym):
+    want, tt, dag = wanted(sym)
+    with gpu.Graph.from_csr(sym.rowptr, sym.col, use_dag=False) as g:
+        for k, w in want.items():
+            assert g.count(k) == w, k
+        for k, p in PLAIN.items():  # the accounting pass recounts as well
+            count, st = g.count(k, stats=True)
+            assert (count, st["setop_elements"]) == O.count(p, dag)[:2], k
+            assert sum(g.count_shard(k, s, 3) for s in range(3)) == count, k
+        assert g.count("tailed-triangle", induced=True) == tt
+        assert g.census4()[2] == tt
+        jobs = [(g, k) for k in want] + [(g, "induced:tailed-triangle"), (g, "k-clique:7")]
+        got = gpu.batch_count(jobs)[0]
+        assert got[:-1] == list(want.values()) + [tt]
+        assert got[-1] == g.count("k-clique:7")
+
+
+@pytest.mark.parametrize("sizes", [(), (33,), (34,), (33, 34, 40), (64,), (65,), (66,), (20,) * 40])
+def test_planted_cliques(gpu, sizes):
+    check(gpu, sparse_with_cliques(30000, sizes, len(sizes)))
+
+
+@pytest.mark.parametrize("n,ef,a,b", [(300, 3, .45, .1375), (2500, 16, .45, .1375),
+                                      (2500, 32, .45, .1375), (50000, 4, .45, .1375),
+                                      (20000, 10, .45, .2391), (9000, 16, .5, .125)])
+def test_weakly_skewed(gpu, n, ef, a, b):
+    check(gpu, O.rmat_graph(n, ef, a, b, b, n))
