@@ -150,6 +150,28 @@ __device__ __forceinline__ acc_t task_groups_k(const JobDesc& j, int64_t b, int6
   }
 }
 
+template <int K, bool PAIRS, bool TT = false>
+__device__ __forceinline__ acc_t task_scan(const JobDesc& j, int64_t b, int64_t e, ScanSmem* sm) {
+  const int warp = threadIdx.x >> 5;
+  acc_t cnt = 0, el = 0;
+  for (int64_t r = b + warp; r < e; r += 8)
+    cnt += scan_root<K, false, PAIRS, PAIRS, TT>(j.dag, j.roots[r], sm + warp, j.tri, el);
+  return cnt;
+}
+
+__device__ __forceinline__ acc_t task_scan_k(const JobDesc& j, int64_t b, int64_t e, ScanSmem* sm) {
+  if (j.kind == kJobDiamond) return task_scan<3, true>(j, b, e, sm);
+  if (j.kind == kJobIndTT) return task_scan<4, true, true>(j, b, e, sm);
+  switch (j.k) {
+    case 3: return task_scan<3, false>(j, b, e, sm);
+    case 4: return task_scan<4, false>(j, b, e, sm);
+    case 5: return task_scan<5, false>(j, b, e, sm);
+    case 6: return task_scan<6, false>(j, b, e, sm);
+    case 7: return task_scan<7, false>(j, b, e, sm);
+    default: return task_scan<8, false>(j, b, e, sm);
+  }
+}
+
 // The warps take the task's roots one at a time from a shared counter (zero at task start),
 // so a warp that drew cheap roots does not wait at the next task fetch for one that drew dear
 // ones.
@@ -371,6 +393,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchArgs a) {
 __global__ void __launch_bounds__(256, 4) k_batch_groups(BatchArgs a) {
   __shared__ uint32_t rows[256];
   __shared__ int degs[256];
+  __shared__ ScanSmem scans[8];
   __shared__ unsigned long long s_task;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -387,6 +410,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_groups(BatchArgs a) {
       case kTaskGroup4: c = task_groups_k<4>(j, t.b, t.e, rows, degs); break;
       case kTaskGroup8: c = task_groups_k<8>(j, t.b, t.e, rows, degs); break;
       case kTaskGroup16: c = task_groups_k<16>(j, t.b, t.e, rows, degs); break;
+      case kTaskScanRoots: c = task_scan_k(j, t.b, t.e, scans); break;
       default: c = task_groups_k<32>(j, t.b, t.e, rows, degs); break;
     }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
@@ -538,10 +562,15 @@ int build_tasks(const std::vector<BatchJobIn>& in, const jgpm_tuning& tu, BatchC
     const int64_t stop = t.deg_begin[per_arc ? 1 : jd.k - 2];
     // roots by out-degree: > 2048 large | (512, 2048] wide | (split, 512] CTA |
     // (32, split] warp | <= 32 groups
-    const int64_t wide_begin = std::min(stop, t.le_begin[5]);
-    const int64_t large_end = std::min(stop, tier_begin(t, kBatchCtaMaxDeg));
-    const int64_t cta_end = std::min(stop, std::max(large_end, tier_begin(t, split)));
+    int64_t wide_begin = std::min(stop, t.le_begin[5]);
+    int64_t large_end = std::min(stop, tier_begin(t, kBatchCtaMaxDeg));
+    int64_t cta_end = std::min(stop, std::max(large_end, tier_begin(t, split)));
     const int64_t warp_end = std::min(stop, std::max(cta_end, t.deg_begin[32]));
+    if (t.light) {
+      add_range_tasks(light, job, kTaskScanRoots, 0, warp_end, 8);
+      wide_begin = large_end = 0;
+      cta_end = warp_end;
+    }
     for (int64_t r = 0; r < wide_begin; ++r) heavy.push_back(make_task(job, kTaskLargeRoot, r, r + 1));
     if (wide_begin > 0) {
       o->any_large = true;
@@ -553,9 +582,9 @@ int build_tasks(const std::vector<BatchJobIn>& in, const jgpm_tuning& tu, BatchC
       o->wdmax = std::max(o->wdmax, std::min(g->max_out_degree, kBatchWideMaxDeg));
     // CTA roots above out-degree 256 count 16-word masks, the others 8-word ones
     const int64_t cta16_end = std::min(cta_end, std::max(large_end, tier_begin(t, 256)));
-    for (int64_t r = large_end; r < cta_end; ++r)
+    for (int64_t r = t.light ? cta_end : large_end; r < cta_end; ++r)
       cta.push_back(make_task(job, r < cta16_end ? kTaskCtaRoot : kTaskCtaRoot8, r, r + 1));
-    if (cta_end > large_end)
+    if (cta_end > large_end && !t.light)
       o->dmax = std::max(o->dmax, std::min(g->max_out_degree, kBatchCtaMaxDeg));
     add_range_tasks(warp, job, kTaskWarpRoots, cta_end, warp_end, std::max<int64_t>(8, rpt / 4));
     // lane groups for d <= 32

@@ -66,7 +66,9 @@ static TierPlan make_plan(const RootTiers& t, int k, int64_t root_begin, int64_t
                           int min_group, int split, int shard, int nshards) {
   const int64_t stop = std::min(root_end, t.deg_begin[k - 2 >= 0 ? k - 2 : 0]);
   auto cut = [&](int64_t b, int64_t e) {
-    TierRange r{std::max(b, root_begin), std::min(e, stop)};
+    TierRange r;
+    r.b = std::max(b, root_begin);
+    r.e = std::min(e, stop);
     return r;
   };
   TierPlan p;
@@ -82,6 +84,10 @@ static TierPlan make_plan(const RootTiers& t, int k, int64_t root_begin, int64_t
   p.mid[1] = cut(b512, b256);
   p.mid[2] = cut(b256, wb);
   p.warp = cut(wb, t.mid_end);
+  if (t.light) {
+    p = TierPlan{};
+    p.scan = cut(0, t.mid_end);
+  }
   // small tier [mid_end, small_end): d in (16,32] -> G32, (8,16] -> G16, (4,8] -> G8, <=4 -> G4
   const int64_t b16 = min_group <= 16 ? t.deg_begin[16] : t.small_end;
   const int64_t b8 = min_group <= 8 ? t.deg_begin[8] : t.small_end;
@@ -94,11 +100,13 @@ static TierPlan make_plan(const RootTiers& t, int k, int64_t root_begin, int64_t
     // shard s of n takes tier indices b + s, b + s + n, ... of every range, so each shard gets
     // an equal share of every out-degree band
     TierRange* all[] = {&p.large, &p.wide, &p.mid[0], &p.mid[1], &p.mid[2], &p.warp,
-                        &p.g32, &p.g16, &p.g8, &p.g4};
+                        &p.g32, &p.g16, &p.g8, &p.g4, &p.scan};
     for (TierRange* r : all) {
       const int64_t b = r->b + shard;
       const int64_t cnt = b < r->e ? (r->e - b + nshards - 1) / nshards : 0;
-      *r = TierRange{b, b + cnt, nshards};
+      r->b = b;
+      r->e = b + cnt;
+      r->step = nshards;
     }
   }
   return p;

@@ -635,6 +635,102 @@ __device__ __forceinline__ int row_members(const uint32_t* Ri, int w_d, uint16_t
   return c;
 }
 
+// One root of out-degree d <= kLightOutDegree of a graph without a rank DAG, on one warp: its rows
+// are scanned four at a time and looked up in the list in shared memory.
+struct ScanSmem {
+  int L[kLightOutDegree];
+  int deg[kLightOutDegree];  // out-degrees (accounting) or hits per list entry (ETRI)
+  uint32_t R[kLightOutDegree * 2];
+};
+template <int K, bool STATS, bool ETRI, bool PAIRS = false, bool TT = false>
+__device__ __forceinline__ acc_t scan_root(const RankDag& g, vid_t u, ScanSmem* sm, uint32_t* tri,
+                                           acc_t& elems) {
+  static_assert(kLightOutDegree == 64, "two list entries and two row elements a lane");
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  const eid_t base = g.rp[u];
+  const int d = (int)(g.rp[u + 1] - base);
+  vid_t L[2];
+  eid_t s[2];
+  int len[2];
+  __syncwarp();  // the last root's readers are done
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    const int j = 32 * b + lane;
+    L[b] = j < d ? __ldg(g.col + base + j) : INT32_MAX;
+    s[b] = j < d ? g.rp[L[b]] : 0;
+    len[b] = j < d ? (int)(g.rp[L[b] + 1] - s[b]) : 0;
+    sm->L[j] = L[b];
+    sm->deg[j] = STATS ? len[b] : 0;
+    sm->R[2 * j] = sm->R[2 * j + 1] = 0u;
+  }
+  __syncwarp();
+  acc_t cnt = 0, pairs = 0, tt = 0;
+  for (int i0 = 0; i0 < d; i0 += U) {
+    eid_t e[U][2];
+    vid_t x[U][2];
+#pragma unroll
+    for (int t = 0; t < U; ++t) {
+      const int i = i0 + t;
+      const int ln = i < d ? __shfl_sync(kFull, i < 32 ? len[0] : len[1], i & 31) : 0;
+      const eid_t si = __shfl_sync(kFull, i < 32 ? s[0] : s[1], i & 31);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        e[t][h] = si + 32 * h + lane;
+        x[t][h] = 32 * h + lane < ln ? __ldg(g.col + e[t][h]) : -1;
+      }
+    }
+    unsigned old[U][2];
+#pragma unroll
+    for (int t = 0; t < U; ++t) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        old[t][h] = 0u;
+        int p = 0;
+#pragma unroll
+        for (int step = 32; step > 0; step >>= 1)
+          if (sm->L[p + step - 1] < x[t][h]) p += step;
+        if (x[t][h] < 0 || sm->L[p] != x[t][h]) continue;
+        if (ETRI) {
+          old[t][h] = atomicAdd(tri + e[t][h], 1u);
+          atomicAdd(&sm->deg[p], 1);
+        }
+        if (K == 3) ++cnt;
+        atomicOr(&sm->R[2 * (i0 + t) + (p >> 5)], 1u << (p & 31));
+      }
+    }
+    if (PAIRS) {
+#pragma unroll
+      for (int t = 0; t < U; ++t) pairs += (acc_t)old[t][0] + (acc_t)old[t][1];
+    }
+  }
+  __syncwarp();
+  if (K > 3) {
+    for (int i = lane; i < d; i += 32) {
+      const uint32_t m[2] = {sm->R[2 * i], sm->R[2 * i + 1]};
+      cnt += RowCount<(K > 3 ? K - 3 : 1), 2, STATS>::run(m, sm->R, 2, sm->deg, elems, 2);
+    }
+  }
+  if (ETRI) {  // the root's own arcs, as in group_root
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = 32 * b + lane;
+      const unsigned rowc = (unsigned)(__popc(sm->R[2 * i]) + __popc(sm->R[2 * i + 1]));
+      const unsigned colc = (unsigned)sm->deg[i], tu = rowc + colc;
+      if (i < d && tu) {
+        const unsigned o = atomicAdd(tri + base + i, tu);
+        if (PAIRS) pairs += pair_gain(o, tu);
+        if (TT) {
+          const acc_t di = tt_deg(g, L[b]);
+          tt += (acc_t)rowc * (tt_deg(g, u) + di) + (acc_t)colc * di;
+        }
+      }
+    }
+  }
+  if (TT) return 12ull * cnt - 4ull * pairs + tt;
+  return PAIRS ? pairs : cnt;
+}
+
 // ---------------------------------------------------------------- warp per root
 // One root of out-degree 32 < d <= kWarpMaxDeg per warp, with the warp's own slice of shared
 // memory (no CTA barriers).

@@ -33,7 +33,7 @@ constexpr int kMaxLevels = 6;  // list tier: candidate lists per warp
 
 // Tier indices b, b + step, ..., (e - b) of them.
 struct TierRange {
-  int64_t b, e;
+  int64_t b = 0, e = 0;
   int64_t step = 1;
   bool empty() const { return e <= b; }
 };
@@ -48,6 +48,7 @@ __device__ __forceinline__ vid_t root_at(const CliqueArgs& a, int64_t i) {
 // out-degree (512, 1024], (256, 512] and (split, 256].
 struct TierPlan {
   TierRange large, wide, mid[3], warp, g32, g16, g8, g4;
+  TierRange scan;  // all roots above 32, of a graph without a rank DAG
 };
 
 // CTAs and global row words of a wide/global-row band of out-degree <= dmax: at most
@@ -179,6 +180,25 @@ __global__ void __launch_bounds__(256, 4) k_clique_warp(CliqueArgs a) {
     if (idx >= a.end) break;
     next = fetch();
     cnt += warp_root<K, STATS, ETRI, PAIRS, TT>(a.dag, root_at(a, idx), ws, a.tri, elems);
+  }
+  add_result<STATS>(a.ctl, cnt, elems);
+  pdl_close();
+}
+
+// --------------------------------- roots above 32 of a graph without a rank DAG, one per warp
+template <int K, bool STATS, bool ETRI = false, bool PAIRS = false, bool TT = false>
+__global__ void __launch_bounds__(256) k_clique_scan(CliqueArgs a) {
+  __shared__ ScanSmem sm[8];
+  const int lane = threadIdx.x & 31;
+  pdl_open();
+  acc_t cnt = 0, elems = 0;
+  for (;;) {
+    unsigned long long c = 0;
+    if (lane == 0) c = atomicAdd(&a.ctl->counter[a.cursor], 1ull);
+    const int64_t idx = a.begin + (int64_t)__shfl_sync(kFull, c, 0);
+    if (idx >= a.end) break;
+    cnt += scan_root<K, STATS, ETRI, PAIRS, TT>(a.dag, root_at(a, idx), &sm[threadIdx.x >> 5],
+                                                a.tri, elems);
   }
   add_result<STATS>(a.ctl, cnt, elems);
   pdl_close();
@@ -435,6 +455,17 @@ int launch_plan_k(const CliqueArgs& base, const TierPlan& p, int sms, cudaStream
     const int64_t grid = std::min<int64_t>((int64_t)sms * per_sm, (a.end - a.begin + 7) / 8);
     const cudaError_t rc =
         tier_launch(pdl(), k_clique_warp<K, STATS, ETRI, PAIRS, TT>, (int)grid, sm, s, a);
+    ++n;
+    if (launch_failed(&err, rc)) return -1;
+  }
+  if (!p.scan.empty()) {
+    a.begin = p.scan.b;
+    a.end = p.scan.e;
+    a.step = p.scan.step;
+    a.cursor = 7;
+    const int64_t grid = std::min<int64_t>((int64_t)sms * 4, (a.end - a.begin + 7) / 8);
+    const cudaError_t rc =
+        tier_launch(pdl(), k_clique_scan<K, STATS, ETRI, PAIRS, TT>, (int)grid, 0, s, a);
     ++n;
     if (launch_failed(&err, rc)) return -1;
   }

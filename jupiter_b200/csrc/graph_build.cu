@@ -338,25 +338,32 @@ __global__ void k_orient_scatter(const int32_t* col, const uint32_t* keep, const
   }
 }
 
-// Row pointers of the DAG and its largest out-degree.  words = words of keep; total = DAG arcs.
+// Row pointers of the DAG; out[0] = its largest out-degree, out[1] = its vertices of out-degree above
+// 32 (both zero before).  words = words of keep; total = DAG arcs.
 __global__ void k_dag_rowptr(const int64_t* rowptr, const uint32_t* keep, const int64_t* pos,
                              int32_t n, int64_t m, int64_t total, int64_t* dag_rowptr,
-                             int* max_out) {
+                             int* out) {
   auto at = [&](int64_t k) {
     return k < m ? pos[k >> 5] + __popc(keep[k >> 5] & ((1u << (k & 31)) - 1u)) : total;
   };
-  int most = 0;
+  int most = 0, over = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += stride) {
     const int64_t b = rowptr[v], p = at(b);
     dag_rowptr[v] = p;
     if (v < n) {
       const int64_t e = rowptr[v + 1];
-      if (e > b) most = max(most, (int)(at(e) - p));
+      const int d = e > b ? (int)(at(e) - p) : 0;
+      most = max(most, d);
+      over += d > 32 ? 1 : 0;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(kAll, most, o));
-  if ((threadIdx.x & 31) == 0 && most) atomicMax(max_out, most);
+  most = (int)__reduce_max_sync(kAll, (unsigned)most);
+  over = (int)__reduce_add_sync(kAll, (unsigned)over);
+  if ((threadIdx.x & 31) == 0 && most) {
+    atomicMax(out, most);
+    if (over) atomicAdd(out + 1, over);
+  }
 }
 
 __global__ void k_max_degree(const int64_t* rowptr, int32_t n, int* out) {
@@ -740,8 +747,8 @@ int ensure_dag(jgpm_graph* g) {
   uint32_t* keep = (uint32_t*)masks.p;
   int32_t* count = (int32_t*)keep + words;
   if ((rc = dalloc((int64_t**)&pos.p, words + 1, s))) return rc;
-  if ((rc = dalloc((int**)&st.p, 1, s))) return rc;
-  JGPM_CUDA_TRY(cudaMemsetAsync(st.p, 0, sizeof(int), s));
+  if ((rc = dalloc((int**)&st.p, 2, s))) return rc;
+  JGPM_CUDA_TRY(cudaMemsetAsync(st.p, 0, 2 * sizeof(int), s));
   JGPM_CUDA_TRY(cudaMemsetAsync(count + words, 0, 4, s));
   if (words > 0 && !have) {
     ArcOwners own;
@@ -765,31 +772,46 @@ int ensure_dag(jgpm_graph* g) {
                                                         (int64_t*)pos.p, n, m, total,
                                                         (int64_t*)rowptr.p, (int*)st.p);
   JGPM_CUDA_TRY(cudaGetLastError());
-  int h = 0;
-  JGPM_CUDA_TRY(cudaMemcpyAsync(&h, st.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int h[2] = {0, 0};
+  JGPM_CUDA_TRY(cudaMemcpyAsync(h, st.p, sizeof(h), cudaMemcpyDeviceToHost, s));
   JGPM_CUDA_TRY(cudaStreamSynchronize(s));
   g->m_dag = total;
-  g->max_out_degree = h;
+  g->max_out_degree = h[0];
+  g->over32 = h[1];
   rowptr.publish(&g->d_dag_rowptr);
   col.publish(&g->d_dag_col);
   return JGPM_OK;
 }
 
-// out[x] for x = 0..33, then thresholds 64, 128, 256, 512, 1024, 2048, 4096: the first index
-// of the descending keys[0..n) whose key is <= the threshold.
-__global__ void k_tier_bounds(const uint32_t* keys, int32_t n, int64_t* out) {
-  const int t = threadIdx.x;
-  if (t >= 41) return;
-  const uint32_t big[7] = {64u, 128u, 256u, 512u, (uint32_t)kMidMaxDeg, 2048u,
-                           (uint32_t)kWideMaxDeg};
-  const uint32_t x = t < 34 ? (uint32_t)t : big[t - 34];
-  int64_t lo = 0, hi = n;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (keys[mid] > x) lo = mid + 1;
-    else hi = mid;
-  }
-  out[t] = lo;
+// Out-degree classes of the tier boundaries: class t holds the out-degrees up to tier_threshold(t)
+// that no lower class holds; the last class the rest.
+constexpr int kTierClasses = 34 + 8;
+constexpr size_t kTierBytes = 256;  // their counters
+__host__ __device__ __forceinline__ int tier_class(int64_t d) {
+  if (d <= 33) return (int)d;
+  int t = 34;
+  for (int64_t top = 64; t < kTierClasses - 1 && d > top; top *= 2) ++t;
+  return t;
+}
+static_assert(kTierClasses * 4 <= kTierBytes && kMidMaxDeg == 1024 && kWideMaxDeg == 4096,
+              "classes 34.. end at 64, 128, 256, 512, 1024, 2048 and 4096");
+
+// Adds up the classes of a CTA's vertices (every thread calls it, once, with its own count array
+// in shared memory zeroed).
+__device__ __forceinline__ void add_classes(const int* mine, int32_t* classes) {
+  __syncthreads();
+  for (int t = threadIdx.x; t < kTierClasses; t += blockDim.x)
+    if (mine[t]) atomicAdd(classes + t, mine[t]);
+}
+
+// Roots of a class above t: the first index of the descending root list that is at or below it.
+// By one warp.
+__device__ __forceinline__ int64_t tier_begin(const int32_t* classes, int t) {
+  const int lane = threadIdx.x & 31;
+  const unsigned a = lane > t ? (unsigned)classes[lane] : 0u;
+  const unsigned b =
+      lane + 32 > t && lane + 32 < kTierClasses ? (unsigned)classes[lane + 32] : 0u;
+  return (int64_t)__reduce_add_sync(kAll, a + b);
 }
 
 // ------------------------------------------------------------------- rank DAG
@@ -800,17 +822,53 @@ __global__ void k_tier_bounds(const uint32_t* keys, int32_t n, int64_t* out) {
 // bitmap on the way.
 namespace {
 
-__global__ void k_degree_keys(const int64_t* rowptr, int32_t n, uint32_t* keys, int32_t* vals) {
+// Sort input of the root list on the id DAG: out-degrees and ids; with them the symmetric degrees
+// and the out-degree classes.
+__global__ void k_root_keys(const int64_t* dag_rowptr, const int64_t* rowptr, int32_t n,
+                            uint32_t* keys, int32_t* vals, int32_t* sdeg, int32_t* classes) {
+  __shared__ int mine[kTierClasses];
+  for (int t = threadIdx.x; t < kTierClasses; t += blockDim.x) mine[t] = 0;
+  __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
-    keys[v] = (uint32_t)(rowptr[v + 1] - rowptr[v]);
+    const int64_t d = dag_rowptr[v + 1] - dag_rowptr[v];
+    keys[v] = (uint32_t)d;
     vals[v] = (int32_t)v;
+    sdeg[v] = (int32_t)(rowptr[v + 1] - rowptr[v]);
+    atomicAdd(&mine[tier_class(d)], 1);
   }
+  add_classes(mine, classes);
+}
+
+// Sort input of the rank DAG: every vertex by its degree.  both: n entries more, with the bit above
+// the others set, for every vertex by descending (out-degree, degree, id), so that one ascending
+// sort gives both orders; deg_bits and out_bits hold the largest degree and out-degree.
+__global__ void k_order_keys(const int64_t* rowptr, const int64_t* dag_rowptr, int32_t n,
+                             int deg_bits, int out_bits, bool both, uint32_t* keys, int32_t* vals,
+                             int32_t* classes) {
+  __shared__ int mine[kTierClasses];
+  for (int t = threadIdx.x; t < kTierClasses; t += blockDim.x) mine[t] = 0;
+  __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+    const uint32_t d = (uint32_t)(dag_rowptr[v + 1] - dag_rowptr[v]);
+    const uint32_t deg = (uint32_t)(rowptr[v + 1] - rowptr[v]);
+    keys[v] = deg;
+    vals[v] = (int32_t)v;
+    if (both) {
+      const uint32_t top = (2u << out_bits) - 1u;  // the bit, and all ones for an out-degree of 0
+      const int64_t at = 2 * (int64_t)n - 1 - v;
+      keys[at] = ((top - d) << deg_bits) | (((1u << deg_bits) - 1u) - deg);
+      vals[at] = (int32_t)v;
+    }
+    atomicAdd(&mine[tier_class(d)], 1);
+  }
+  add_classes(mine, classes);
 }
 
 // order[p] = the vertex at position p of the ascending (degree, id) order; its new id is
-// n - 1 - p.  outdeg gets a zero at index n (the end of the row-pointer scan).  keys and vals are
-// the root list's sort input: out-degrees and new ids.
+// n - 1 - p.  outdeg gets a zero at index n (the end of the row-pointer scan).  keys and vals (may
+// be null): the sort input for the vertices by out-degree, in the order of the new ids.
 __global__ void k_rank_label(const int32_t* order, const int64_t* dag_rowptr,
                              const int64_t* rowptr, int32_t n, int32_t* newid, int64_t* outdeg,
                              int32_t* sdeg, uint32_t* keys, int32_t* vals) {
@@ -821,15 +879,17 @@ __global__ void k_rank_label(const int32_t* order, const int64_t* dag_rowptr,
     newid[v] = (int32_t)x;
     const int64_t d = dag_rowptr[v + 1] - dag_rowptr[v];
     outdeg[x] = d;
-    keys[x] = (uint32_t)d;
-    vals[x] = (int32_t)x;
     sdeg[x] = (int32_t)(rowptr[v + 1] - rowptr[v]);
+    if (keys) {
+      keys[x] = (uint32_t)d;
+      vals[x] = v;
+    }
     if (p == 0) outdeg[n] = 0;
   }
 }
 
 // k_rank_label and the row-pointer scan in one launch, for graphs of at most kRankOneCta vertices,
-// whose first count is bound by the number of launches (1,000 vertices: 123 us, now 118 us).
+// whose first count is bound by the number of launches.
 constexpr int32_t kRankOneCta = 8192;
 __global__ void __launch_bounds__(1024)
     k_rank_label_scan(const int32_t* order, const int64_t* dag_rowptr, const int64_t* rowptr,
@@ -845,9 +905,11 @@ __global__ void __launch_bounds__(1024)
     const int64_t d = dag_rowptr[v + 1] - dag_rowptr[v];
     newid[v] = x;
     rp[x] = d;
-    keys[x] = (uint32_t)d;
-    vals[x] = x;
     sdeg[x] = (int32_t)(rowptr[v + 1] - rowptr[v]);
+    if (keys) {
+      keys[x] = (uint32_t)d;
+      vals[x] = v;
+    }
     sum += d;
   }
   int64_t incl = sum;
@@ -900,83 +962,108 @@ __device__ __forceinline__ void bitonic_sort(int32_t* a, int n, int tid, int nth
 }
 
 struct RowArgs {
-  const int32_t* roots;  // rank-DAG ids by descending out-degree
-  const int32_t* order;
+  const int32_t* verts;  // id-DAG vertices by descending out-degree
   const int64_t* dag_rowptr;
   const int32_t* dag_col;
   const int32_t* newid;
   const int64_t* rp;
   int32_t* col;
   uint32_t* bits;
-  int32_t n, h;
+  int32_t* roots;          // receives the new ids of verts
+  const int32_t* classes;  // out-degree classes: where the kernels' ranges of verts begin
+  int32_t h;
 };
 
 __device__ __forceinline__ void set_bit(const RowArgs& a, int32_t x, int32_t w) {
   if (x < a.h) atomicOr(a.bits + rank_bits_row((uint32_t)x) + ((uint32_t)w >> 5), 1u << (w & 31));
 }
 
-// Rows of out-degree 1..G, one per group of G lanes, sorted in registers.
+// Rows of out-degree 1..G, one per group of G lanes, sorted in registers; kRowsAhead at a time, so
+// that their chains of gathers (vertex, row, arcs, new ids) overlap: one task at a time took 380 us
+// on 16.7 M arcs of 4,194,304 vertices.
+constexpr int kRowsAhead = 4;
 template <int G>
 __device__ __forceinline__ void rank_rows_group(const RowArgs& a, int64_t b, int64_t e,
                                                 int64_t task) {
+  constexpr int U = kRowsAhead;
   const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-  const int64_t idx = b + task * (32 / G) + lane / G;
-  int32_t x = -1;
-  int64_t s = 0, o = 0;
-  int d = 0;
-  if (idx < e) {
-    x = a.roots[idx];
-    s = a.dag_rowptr[a.order[a.n - 1 - x]];
-    o = a.rp[x];
-    d = (int)(a.rp[x + 1] - o);
+  int32_t v[U], x[U], key[U];
+  int64_t s[U], o[U];
+  int d[U];
+#pragma unroll
+  for (int q = 0; q < U; ++q) {
+    const int64_t idx = b + (task * U + q) * (32 / G) + lane / G;
+    v[q] = idx < e ? a.verts[idx] : -1;
   }
-  int32_t key = gl < d ? a.newid[a.dag_col[s + gl]] : INT32_MAX;
 #pragma unroll
-  for (int k = 2; k <= G; k <<= 1) {
+  for (int q = 0; q < U; ++q) {
+    const bool in = v[q] >= 0;
+    x[q] = in ? a.newid[v[q]] : -1;
+    s[q] = in ? a.dag_rowptr[v[q]] : 0;
+    d[q] = in ? (int)(a.dag_rowptr[v[q] + 1] - s[q]) : 0;
+  }
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const int32_t other = __shfl_xor_sync(0xffffffffu, key, j);
-      const bool up = (gl & k) == 0, low = (gl & j) == 0;
-      key = (up == low) ? min(key, other) : max(key, other);
+  for (int q = 0; q < U; ++q) {
+    const int64_t idx = b + (task * U + q) * (32 / G) + lane / G;
+    o[q] = x[q] >= 0 ? a.rp[x[q]] : 0;
+    if (x[q] >= 0 && gl == 0) a.roots[idx] = x[q];
+    key[q] = gl < d[q] ? a.dag_col[s[q] + gl] : -1;
+  }
+#pragma unroll
+  for (int q = 0; q < U; ++q) key[q] = key[q] >= 0 ? a.newid[key[q]] : INT32_MAX;
+#pragma unroll
+  for (int q = 0; q < U; ++q) {
+#pragma unroll
+    for (int k = 2; k <= G; k <<= 1) {
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const int32_t other = __shfl_xor_sync(0xffffffffu, key[q], j);
+        const bool up = (gl & k) == 0, low = (gl & j) == 0;
+        key[q] = (up == low) ? min(key[q], other) : max(key[q], other);
+      }
+    }
+    if (gl < d[q]) {
+      a.col[o[q] + gl] = key[q];
+      set_bit(a, x[q], key[q]);
     }
   }
-  if (gl < d) {
-    a.col[o + gl] = key;
-    set_bit(a, x, key);
+}
+
+// Vertices of out-degree 17..32 | 9..16 | 5..8 | 1..4.
+__global__ void k_rank_rows_small(RowArgs a) {
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t b[5] = {tier_begin(a.classes, 32), tier_begin(a.classes, 16),
+                        tier_begin(a.classes, 8), tier_begin(a.classes, 4),
+                        tier_begin(a.classes, 0)};
+  int64_t end[4], n = 0;  // end of each range's tasks
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int per = kRowsAhead << q;
+    n += (b[q + 1] - b[q] + per - 1) / per;
+    end[q] = n;
+  }
+  for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += warps) {
+    if (t < end[0]) rank_rows_group<32>(a, b[0], b[1], t);
+    else if (t < end[1]) rank_rows_group<16>(a, b[1], b[2], t - end[0]);
+    else if (t < end[2]) rank_rows_group<8>(a, b[2], b[3], t - end[1]);
+    else rank_rows_group<4>(a, b[3], b[4], t - end[2]);
   }
 }
 
-// Roots of out-degree 17..32 | 9..16 | 5..8 | 1..4, whose ranges follow from the tier boundaries on
-// the device (k_tier_bounds), so that the launch needs no read-back first.
-__global__ void k_rank_rows_small(RowArgs a, const int64_t* bounds) {
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  struct {
-    int64_t b[5];
-  } r = {{bounds[32], bounds[16], bounds[8], bounds[4], bounds[0]}};
-  int64_t n[4];
-  n[0] = r.b[1] - r.b[0];
-  n[1] = (r.b[2] - r.b[1] + 1) / 2;
-  n[2] = (r.b[3] - r.b[2] + 3) / 4;
-  n[3] = (r.b[4] - r.b[3] + 7) / 8;
-  const int64_t total = n[0] + n[1] + n[2] + n[3];
-  for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += warps) {
-    if (t < n[0]) rank_rows_group<32>(a, r.b[0], r.b[1], t);
-    else if (t < n[0] + n[1]) rank_rows_group<16>(a, r.b[1], r.b[2], t - n[0]);
-    else if (t < n[0] + n[1] + n[2]) rank_rows_group<8>(a, r.b[2], r.b[3], t - n[0] - n[1]);
-    else rank_rows_group<4>(a, r.b[3], r.b[4], t - n[0] - n[1] - n[2]);
-  }
-}
+constexpr int kClassMid = 38;  // the class that ends at kMidMaxDeg
 
 // Rows of out-degree 33..kMidMaxDeg, one per warp, sorted in the warp's slice of shared memory.
-__global__ void __launch_bounds__(256) k_rank_rows_warp(RowArgs a, int64_t b, int64_t e) {
+__global__ void __launch_bounds__(256) k_rank_rows_warp(RowArgs a) {
   __shared__ int32_t buf[8][kMidMaxDeg];
   int32_t* k = buf[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t b = tier_begin(a.classes, kClassMid), e = tier_begin(a.classes, 32);
   for (int64_t q = b + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); q < e; q += warps) {
-    const int32_t x = a.roots[q];
-    const int64_t s = a.dag_rowptr[a.order[a.n - 1 - x]], o = a.rp[x];
-    const int d = (int)(a.rp[x + 1] - o);
+    const int32_t v = a.verts[q], x = a.newid[v];
+    const int64_t s = a.dag_rowptr[v], o = a.rp[x];
+    const int d = (int)(a.dag_rowptr[v + 1] - s);
+    if (lane == 0) a.roots[q] = x;
     for (int t = lane; t < d; t += 32) k[t] = a.newid[a.dag_col[s + t]];
     __syncwarp();
     bitonic_sort(k, d, lane, 32, [] { __syncwarp(); });
@@ -990,13 +1077,15 @@ __global__ void __launch_bounds__(256) k_rank_rows_warp(RowArgs a, int64_t b, in
 
 // Longer rows, one per CTA: in shared memory up to kRankCtaRow entries, else in place.
 constexpr int kRankCtaRow = 4096;
-__global__ void __launch_bounds__(1024) k_rank_rows_cta(RowArgs a, int64_t b, int64_t e) {
+__global__ void __launch_bounds__(1024) k_rank_rows_cta(RowArgs a) {
   __shared__ int32_t buf[kRankCtaRow];
-  for (int64_t q = b + blockIdx.x; q < e; q += gridDim.x) {
-    const int32_t x = a.roots[q];
-    const int64_t s = a.dag_rowptr[a.order[a.n - 1 - x]], o = a.rp[x];
-    const int d = (int)(a.rp[x + 1] - o);
+  const int64_t e = tier_begin(a.classes, kClassMid);
+  for (int64_t q = blockIdx.x; q < e; q += gridDim.x) {
+    const int32_t v = a.verts[q], x = a.newid[v];
+    const int64_t s = a.dag_rowptr[v], o = a.rp[x];
+    const int d = (int)(a.dag_rowptr[v + 1] - s);
     int32_t* k = d <= kRankCtaRow ? buf : a.col + o;
+    if (threadIdx.x == 0) a.roots[q] = x;
     for (int t = threadIdx.x; t < d; t += blockDim.x) k[t] = a.newid[a.dag_col[s + t]];
     __syncthreads();
     bitonic_sort(k, d, threadIdx.x, blockDim.x, [] { __syncthreads(); });
@@ -1043,101 +1132,148 @@ int32_t rank_top(int32_t n, int64_t m_dag) {
 
 size_t rank_bits_words(int32_t h) { return (size_t)rank_bits_row((uint32_t)h); }
 
+// The tier boundaries from the out-degree classes, brought back to the host (waits for the stream,
+// so the structures queued before it are complete: batches and server slots read them on streams
+// of their own).
+int read_tiers(jgpm_graph* g, const int32_t* classes) {
+  int32_t c[kTierClasses];
+  JGPM_CUDA_TRY(cudaMemcpyAsync(c, classes, sizeof(c), cudaMemcpyDeviceToHost, g->stream));
+  JGPM_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  int64_t first[kTierClasses];  // roots above each class
+  int64_t above = 0;
+  for (int t = kTierClasses - 1; t >= 0; --t) {
+    first[t] = above;
+    above += c[t];
+  }
+  RootTiers& t = g->tiers;
+  for (int x = 0; x < 34; ++x) t.deg_begin[x] = first[x];
+  t.small_end = first[0];
+  t.mid_end = first[32];
+  t.large_end = first[38];   // d <= kMidMaxDeg
+  t.wide_begin = first[40];  // d <= kWideMaxDeg
+  const int le[6] = {32, 34, 35, 36, 37, 39};  // 32, 64, 128, 256, 512, 2048
+  for (int x = 0; x < 6; ++x) t.le_begin[x] = first[le[x]];
+  return JGPM_OK;
+}
+
+int bits_for(int32_t most) { return std::max(1, 32 - __builtin_clz((unsigned)std::max(1, most))); }
+
+// The tiers of a graph whose out-degrees are all small, on the id DAG.
+int build_light_tiers(jgpm_graph* g) {
+  cudaStream_t s = g->stream;
+  const int32_t n = g->n;
+  int rc;
+  const int out_bits = bits_for(g->max_out_degree);
+  size_t tb = 0;
+  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(
+      nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
+      n, 0, out_bits, s));
+  const size_t vec = ((size_t)n * 4 + 255) & ~(size_t)255;
+  DevBuf buf(s);  // classes, two key arrays, values, cub's space
+  if ((rc = dalloc((char**)&buf.p, kTierBytes + 3 * vec + tb, s))) return rc;
+  char* at = (char*)buf.p + kTierBytes;
+  int32_t* classes = (int32_t*)buf.p;
+  uint32_t *k0 = (uint32_t*)at, *k1 = (uint32_t*)(at + vec);
+  int32_t* v0 = (int32_t*)(at + 2 * vec);
+  if ((rc = dalloc((char**)&g->d_rd_mem, 2 * vec, s))) return rc;
+  g->d_rd_sdeg = (int32_t*)g->d_rd_mem;
+  g->tiers.d_roots = (int32_t*)((char*)g->d_rd_mem + vec);
+  JGPM_CUDA_TRY(cudaMemsetAsync(classes, 0, kTierBytes, s));
+  k_root_keys<<<grid_for(n), 256, 0, s>>>(g->d_dag_rowptr, g->d_rowptr, n, k0, v0, g->d_rd_sdeg,
+                                          classes);
+  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(
+      at + 3 * vec, tb, k0, k1, v0, g->tiers.d_roots, n, 0, out_bits, s));
+  JGPM_CUDA_TRY(cudaGetLastError());
+  g->tiers.light = true;
+  return read_tiers(g, classes);
+}
+
+// Largest graph whose two vertex orders come from one sort of 2n entries: three launches and two
+// memsets less, for up to two passes over the entries more.
+constexpr int32_t kOneSort = 1 << 18;
+// Up to this size a sort is one launch anyway.
+constexpr int32_t kTwoSorts = 4096;
+
 // Renumbers the vertices and sorts the roots: g->d_rd_rowptr, d_rd_sdeg, tiers; then the rows
-// and the bitmap.
+// and the bitmap.  Every range of the kernels follows from the out-degree classes on the device:
+// the host waits once, at the end.
 int build_rank_dag(jgpm_graph* g) {
   cudaStream_t s = g->stream;
   const int32_t n = g->n;
   int rc;
-  constexpr int kNThr = 34 + 7;  // tier thresholds: 0..33, then 64, 128, 256, 512, 1024, 2048, 4096
-  const int deg_bits = std::max(1, 32 - __builtin_clz((unsigned)std::max(1, g->max_degree)));
-  const int out_bits = std::max(1, 32 - __builtin_clz((unsigned)std::max(1, g->max_out_degree)));
+  const int deg_bits = bits_for(g->max_degree), out_bits = bits_for(g->max_out_degree);
+  const bool both = n > kTwoSorts && n <= kOneSort && deg_bits + out_bits < 32;
+  const int64_t entries = both ? 2 * (int64_t)n : n;
+  const int bits = both ? deg_bits + out_bits + 1 : deg_bits;
   size_t tb = 0, tb2 = 0, tb3 = 0;
   JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr,
                                                 (uint32_t*)nullptr, (int32_t*)nullptr,
-                                                (int32_t*)nullptr, n, 0, deg_bits, s));
-  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(
-      nullptr, tb2, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
-      n, 0, out_bits, s));
+                                                (int32_t*)nullptr, entries, 0, bits, s));
+  if (!both)
+    JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(
+        nullptr, tb2, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
+        (int64_t)n, 0, out_bits, s));
   JGPM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb3, (int64_t*)nullptr, (int64_t*)nullptr,
                                               n + 1, s));
   tb = std::max(tb, std::max(tb2, tb3));
-  // one temporary allocation: two key arrays, values, order, new ids, boundaries, cub's space
-  const size_t vec = ((size_t)n * 4 + 255) & ~(size_t)255;
-  DevBuf buf(s);
-  if ((rc = dalloc((char**)&buf.p, 5 * vec + 512 + tb, s))) return rc;
-  char* at = (char*)buf.p;
-  uint32_t *k0 = (uint32_t*)at, *k1 = (uint32_t*)(at + vec);
-  int32_t *v0 = (int32_t*)(at + 2 * vec), *order = (int32_t*)(at + 3 * vec),
-          *newid = (int32_t*)(at + 4 * vec);
-  int64_t* bnd = (int64_t*)(at + 5 * vec);
-  void* tmp = at + 5 * vec + 512;
-  static_assert(kNThr * 8 <= 512, "tier boundaries");
-  // one allocation (d_rd_rowptr owns it): row pointers, degrees, roots, arcs, bitmap
-  g->rd_h = rank_top(n, g->m_dag);
-  const size_t words = rank_bits_words(g->rd_h);
   auto room = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+  const size_t vec = room((size_t)n * 4), sorted = room((size_t)entries * 4);
+  // one temporary allocation: keys and values, in and out, new ids, vertices by out-degree, cub's
+  // space
+  DevBuf buf(s);
+  if ((rc = dalloc((char**)&buf.p, 4 * sorted + 2 * vec + tb, s))) return rc;
+  char* at = (char*)buf.p;
+  uint32_t *k0 = (uint32_t*)at, *k1 = (uint32_t*)(at + sorted);
+  int32_t *v0 = (int32_t*)(at + 2 * sorted), *order = (int32_t*)(at + 3 * sorted),
+          *newid = (int32_t*)(at + 4 * sorted), *verts = (int32_t*)(at + 4 * sorted + vec);
+  if (both) verts = order + n;
+  void* tmp = at + 4 * sorted + 2 * vec;
+  // one allocation: row pointers, degrees, roots, arcs, bitmap, out-degree classes
+  g->rd_h = rank_top(n, g->m_dag);
+  const size_t bit_bytes = room(rank_bits_words(g->rd_h) * 4);
   const size_t rp_bytes = room(((size_t)n + 1) * 8), arc_bytes = room((size_t)g->m_dag * 4);
-  if ((rc = dalloc((char**)&g->d_rd_rowptr, rp_bytes + 2 * vec + arc_bytes + words * 4, s)))
+  if ((rc = dalloc((char**)&g->d_rd_mem, rp_bytes + 2 * vec + arc_bytes + bit_bytes + kTierBytes,
+                   s)))
     return rc;
-  char* own = (char*)g->d_rd_rowptr + rp_bytes;
+  g->d_rd_rowptr = (int64_t*)g->d_rd_mem;
+  char* own = (char*)g->d_rd_mem + rp_bytes;
   g->d_rd_sdeg = (int32_t*)own;
   g->tiers.d_roots = (int32_t*)(own + vec);
   g->d_rd_col = (int32_t*)(own + 2 * vec);
   g->d_rd_bits = (uint32_t*)(own + 2 * vec + arc_bytes);
-  JGPM_CUDA_TRY(cudaMemsetAsync(g->d_rd_bits, 0, words * 4, s));
-  k_degree_keys<<<grid_for(n), 256, 0, s>>>(g->d_rowptr, n, k0, v0);
-  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, v0, order, n, 0, deg_bits, s));
+  int32_t* classes = (int32_t*)(own + 2 * vec + arc_bytes + bit_bytes);
+  JGPM_CUDA_TRY(cudaMemsetAsync(g->d_rd_bits, 0, bit_bytes + kTierBytes, s));
+  k_order_keys<<<grid_for(n), 256, 0, s>>>(g->d_rowptr, g->d_dag_rowptr, n, deg_bits, out_bits,
+                                           both, k0, v0, classes);
+  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k1, v0, order, entries, 0, bits, s));
+  uint32_t* k2 = both ? nullptr : k0;  // the second sort's input
+  int32_t* v2 = both ? nullptr : v0;
   if (n <= kRankOneCta) {
     k_rank_label_scan<<<1, 1024, 0, s>>>(order, g->d_dag_rowptr, g->d_rowptr, n, newid,
-                                         g->d_rd_rowptr, g->d_rd_sdeg, k0, v0);
+                                         g->d_rd_rowptr, g->d_rd_sdeg, k2, v2);
   } else {
     k_rank_label<<<grid_for(n), 256, 0, s>>>(order, g->d_dag_rowptr, g->d_rowptr, n, newid,
-                                             g->d_rd_rowptr, g->d_rd_sdeg, k0, v0);
+                                             g->d_rd_rowptr, g->d_rd_sdeg, k2, v2);
     JGPM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tb, g->d_rd_rowptr, g->d_rd_rowptr, n + 1,
                                                 s));
   }
-  // root list: keys are out-degrees, sorted over the bits the largest one needs
-  JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, k0, k1, v0, g->tiers.d_roots, n,
-                                                          0, out_bits, s));
-  // keys descending: [>kMidMaxDeg][33..kMidMaxDeg][1..32][0...].  The tier boundaries
-  // (first index with key <= x for each threshold x) are found on the device; only they come
-  // back to the host.
-  k_tier_bounds<<<1, 64, 0, s>>>(k1, n, bnd);
-  const RowArgs a{g->tiers.d_roots, order, g->d_dag_rowptr, g->d_dag_col, newid, g->d_rd_rowptr,
-                  g->d_rd_col, g->d_rd_bits, n, g->rd_h};
-  k_rank_rows_small<<<grid_for((int64_t)n * 4), 256, 0, s>>>(a, bnd);
+  if (!both)
+    JGPM_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, k0, k1, v0, verts, (int64_t)n,
+                                                            0, out_bits, s));
+  const RowArgs a{verts, g->d_dag_rowptr, g->d_dag_col, newid, g->d_rd_rowptr, g->d_rd_col,
+                  g->d_rd_bits, g->tiers.d_roots, classes, g->rd_h};
+  k_rank_rows_small<<<grid_for((int64_t)n * 2), 256, 0, s>>>(a);
+  if (g->max_out_degree > 32)
+    k_rank_rows_warp<<<(int)std::min<int64_t>(148 * 6, ((int64_t)n + 7) / 8), 256, 0, s>>>(a);
+  if (g->max_out_degree > kMidMaxDeg) k_rank_rows_cta<<<148 * 2, 1024, 0, s>>>(a);
   JGPM_CUDA_TRY(cudaGetLastError());
-  int64_t hb[kNThr];
-  JGPM_CUDA_TRY(cudaMemcpyAsync(hb, bnd, sizeof(hb), cudaMemcpyDeviceToHost, s));
-  JGPM_CUDA_TRY(cudaStreamSynchronize(s));
-  RootTiers& t = g->tiers;
-  for (int x = 0; x < 34; ++x) t.deg_begin[x] = hb[x];
-  t.small_end = hb[0];
-  t.mid_end = hb[32];
-  t.large_end = hb[34 + 4];   // d <= kMidMaxDeg
-  t.wide_begin = hb[34 + 6];  // d <= kWideMaxDeg
-  t.le_begin[0] = hb[32];
-  t.le_begin[1] = hb[34 + 0];
-  t.le_begin[2] = hb[34 + 1];
-  t.le_begin[3] = hb[34 + 2];
-  t.le_begin[4] = hb[34 + 3];
-  t.le_begin[5] = hb[34 + 5];
-  if (t.large_end > 0)
-    k_rank_rows_cta<<<(int)std::min<int64_t>(t.large_end, 148 * 2), 1024, 0, s>>>(a, 0,
-                                                                                t.large_end);
-  if (t.mid_end > t.large_end)
-    k_rank_rows_warp<<<grid_for((t.mid_end - t.large_end) * 32), 256, 0, s>>>(a, t.large_end,
-                                                                              t.mid_end);
-  JGPM_CUDA_TRY(cudaGetLastError());
-  // batches and server slots read the rows on streams of their own
-  if (t.mid_end > 0) JGPM_CUDA_TRY(cudaStreamSynchronize(s));
-  return JGPM_OK;
+  return read_tiers(g, classes);
 }
 
 void free_rank_dag(jgpm_graph* g) {
-  gfree(g->d_rd_rowptr, g->stream);  // holds d_rd_sdeg, tiers.d_roots, d_rd_col and d_rd_bits
+  gfree(g->d_rd_mem, g->stream);
   gfree(g->d_rd_rk, g->stream);
+  g->d_rd_mem = nullptr;
   g->d_rd_rowptr = nullptr;
   g->d_rd_col = nullptr;
   g->d_rd_sdeg = nullptr;
@@ -1153,14 +1289,36 @@ int ensure_tiers(jgpm_graph* g) {
   int rc;
   if ((rc = ensure_dag(g))) return rc;
   if (g->tiers.d_roots) return JGPM_OK;
+  if ((rc = light_dag(g) ? build_light_tiers(g) : build_rank_dag(g))) free_rank_dag(g);
+  return rc;
+}
+
+int ensure_rank_dag(jgpm_graph* g) {
+  int rc;
+  if ((rc = ensure_dag(g))) return rc;
+  if (g->d_rd_rowptr) return JGPM_OK;
+  free_rank_dag(g);  // tiers on the id DAG
   if ((rc = build_rank_dag(g))) free_rank_dag(g);
   return rc;
+}
+
+// Graphs that are counted on the id DAG, every row by scans: renumbering them costs more than it
+// saves, where rows are short and few lie in the bitmap.  R-MAT, first call | later calls in us, rank
+// DAG and id DAG: 4-cliques of 40,000 vertices, edge factor 8, a = 0.51: 165 and 122 | 54 and 53; of
+// 4,194,304 vertices, edge factor 4, a = 0.51 (out-degrees up to 44): 1,186 and 767 | 574 and 620.
+// A graph that lies in the bitmap whole, with some 12 arcs a vertex or more, is better off there
+// (2,500 vertices, edge factor 32, a = 0.45: 116 and 88 | 40 and 49), and so are graphs with more
+// roots above 32 entries, whose pairs grow with the square.
+bool light_dag(const jgpm_graph* g) {
+  if (g->max_out_degree > kLightOutDegree || g->over32 > g->m_dag / 2048) return false;
+  return g->m_dag < 12 * (int64_t)g->n || rank_top(g->n, g->m_dag) < g->n;
 }
 
 int ensure_rank_prefix(jgpm_graph* g) {
   if (g->d_rd_rk) return JGPM_OK;
   int rc;
   if ((rc = ensure_tiers(g))) return rc;
+  if (!g->d_rd_rowptr) return JGPM_OK;  // no bitmap
   if ((rc = dalloc(&g->d_rd_rk, rank_bits_words(g->rd_h), g->stream))) return rc;
   k_rank_prefix<<<grid_for((int64_t)g->rd_h * 32), 256, 0, g->stream>>>(g->d_rd_bits, g->rd_h,
                                                                         g->d_rd_rk);
@@ -1171,8 +1329,8 @@ int ensure_rank_prefix(jgpm_graph* g) {
 
 RankDag rank_dag(const jgpm_graph* g) {
   RankDag r;
-  r.rp = g->d_rd_rowptr;
-  r.col = g->d_rd_col;
+  r.rp = g->d_rd_rowptr ? g->d_rd_rowptr : g->d_dag_rowptr;
+  r.col = g->d_rd_rowptr ? g->d_rd_col : g->d_dag_col;
   r.bits = g->d_rd_bits;
   r.rk = g->d_rd_rk;
   r.sdeg = g->d_rd_sdeg;
@@ -1181,7 +1339,7 @@ RankDag rank_dag(const jgpm_graph* g) {
 }
 
 uint64_t rank_dag_bytes(const jgpm_graph* g) {
-  if (!g->d_rd_rowptr) return 0;
+  if (!g->d_rd_rowptr) return g->d_rd_mem ? (uint64_t)g->n * 4 : 0;  // degrees
   const uint64_t words = rank_bits_words(g->rd_h);
   return (uint64_t)(g->n + 1) * 8 + (uint64_t)g->m_dag * 4 + (uint64_t)g->n * 4 + words * 4 +
          (g->d_rd_rk ? words * 2 : 0);

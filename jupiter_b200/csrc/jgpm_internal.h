@@ -26,6 +26,8 @@ struct DevCsr {
 // multiple of 32) the rows are also kept as a bitmap, a lower triangle of words: vertex x has
 // the words rank_bits_row(x) .. + x / 32, bit w set <=> x -> w.  rk[i] is the number of arcs of
 // the row in the words before word i (built for the per-arc counter modes only).
+// Graphs of small out-degrees (light_dag) have none; there this is a view of the id DAG, with
+// h = 0: arcs run either way, rows ascending.
 struct RankDag {
   const eid_t* rp = nullptr;
   const vid_t* col = nullptr;
@@ -49,8 +51,10 @@ constexpr int kMidMaxDeg = 1024;
 // Roots of out-degree kMidMaxDeg < d <= kWideMaxDeg still run on local bitmaps, with the
 // bitmap rows in global scratch; larger ones run on edge-rooted lists.
 constexpr int kWideMaxDeg = 4096;
+// Largest out-degree of a graph that is counted on the id DAG.
+constexpr int kLightOutDegree = 64;
 
-// Roots are rank-DAG ids.
+// Roots are ids of the DAG that rank_dag() gives.
 //   deg_begin[x] = first index whose out-degree is <= x (0 <= x <= 33), so the roots with
 //   d >= k-1 are the prefix [0, deg_begin[k-2]).
 struct RootTiers {
@@ -60,6 +64,7 @@ struct RootTiers {
   // first index with out-degree <= 32, 64, 128, 256, 512, 2048
   int64_t le_begin[6] = {0, 0, 0, 0, 0, 0};
   int64_t wide_begin = 0;  // first index with out-degree <= kWideMaxDeg
+  bool light = false;      // on the id DAG: every root is scanned (light_dag)
 };
 
 struct jgpm_graph_impl;
@@ -92,7 +97,9 @@ struct jgpm_graph {
   uint32_t* d_keep = nullptr;  // arc masks and counts from the validation, until the DAG is built
   int64_t* d_dag_rowptr = nullptr;
   int32_t* d_dag_col = nullptr;
-  // rank DAG (built with the root tiers)
+  // rank DAG (built with the root tiers): one allocation, d_rd_mem, holds it and the roots.
+  // d_rd_rowptr == null with tiers in place: the tiers are on the id DAG (light_dag)
+  void* d_rd_mem = nullptr;
   int64_t* d_rd_rowptr = nullptr;
   int32_t* d_rd_col = nullptr;
   int32_t* d_rd_sdeg = nullptr;
@@ -115,6 +122,7 @@ struct jgpm_graph {
   int64_t c4_ndense = 0;   // large apexes that count in dense arrays (c4_dense_apex)
   std::vector<uint64_t> c4_large_keys;  // host copy: wedge bound of each large apex, descending
   int32_t max_out_degree = 0;
+  int32_t over32 = 0;  // vertices of out-degree above 32
   jgpm::RootTiers tiers;
   // per-graph reusable launch state
   jgpm::DevControl* d_ctl = nullptr;
@@ -180,8 +188,11 @@ int ensure_rank_csr(jgpm_graph* g);
 // c4.cu: apex classes of the 4-cycle count (needs the rank CSR)
 int ensure_c4_apexes(jgpm_graph* g);
 int count_c4_wedge(jgpm_graph* g, uint64_t* out, double* ms);
-// The rank DAG and the root tiers on it.
+// The root tiers, and the DAG they are on: the rank DAG, or the id DAG where light_dag holds.
 int ensure_tiers(jgpm_graph* g);
+bool light_dag(const jgpm_graph* g);
+// The root tiers on the rank DAG, whatever the graph.
+int ensure_rank_dag(jgpm_graph* g);
 // The row prefix counts of the bitmap (RankDag::rk), for the per-arc counter modes.
 int ensure_rank_prefix(jgpm_graph* g);
 RankDag rank_dag(const jgpm_graph* g);

@@ -835,6 +835,7 @@ int run_induced_tt(jgpm_graph* g, uint64_t* out, double* ms) {
 // P5 from per-arc triangle and 4-clique counters in g->d_aux (arc4.cu).
 int run_p5_arcs(jgpm_graph* g, uint64_t* out, double* ms) {
   int rc;
+  if ((rc = ensure_rank_dag(g))) return rc;
   if ((rc = ensure_rank_prefix(g))) return rc;
   if ((rc = ensure_control(g))) return rc;
   if ((rc = ensure_aux(g, arc4_bytes(g->m_dag)))) return rc;
