@@ -274,17 +274,39 @@ __global__ void k_validate(const int64_t* rowptr, const int32_t* col, int32_t n,
   if (lane == 0 && nd) atomicAdd(down, nd);
 }
 
+struct DegreeStats {
+  int most;
+  unsigned long long squares;  // sum of the squared degrees
+};
+
+// Every thread of a full warp calls it.
+__device__ __forceinline__ void add_degree_stats(int most, unsigned long long squares,
+                                                 DegreeStats* out) {
+  for (int o = 16; o > 0; o >>= 1) {
+    most = max(most, __shfl_xor_sync(kAll, most, o));
+    squares += __shfl_xor_sync(kAll, squares, o);
+  }
+  if ((threadIdx.x & 31) == 0 && most) {
+    atomicMax(&out->most, most);
+    atomicAdd(&out->squares, squares);
+  }
+}
+
 __global__ void k_rowptr_check(const int64_t* rowptr, int32_t n, int64_t m, int* bad,
-                               int* max_degree) {
+                               DegreeStats* stats) {
   int most = 0;
+  unsigned long long squares = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     const int64_t d = rowptr[v + 1] - rowptr[v];
-    if (d < 0 || d > INT32_MAX) atomicExch(bad, 1);
-    else most = max(most, (int)d);
+    if (d < 0 || d > INT32_MAX) {
+      atomicExch(bad, 1);
+    } else {
+      most = max(most, (int)d);
+      squares += (unsigned long long)d * (unsigned long long)d;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(kAll, most, o));
-  if ((threadIdx.x & 31) == 0 && most) atomicMax(max_degree, most);
+  add_degree_stats(most, squares, stats);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (rowptr[0] != 0 || rowptr[n] != m) atomicExch(bad, 1);
   }
@@ -366,13 +388,16 @@ __global__ void k_dag_rowptr(const int64_t* rowptr, const uint32_t* keep, const 
   }
 }
 
-__global__ void k_max_degree(const int64_t* rowptr, int32_t n, int* out) {
-  int local = 0;
+__global__ void k_degree_stats(const int64_t* rowptr, int32_t n, DegreeStats* out) {
+  int most = 0;
+  unsigned long long squares = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride)
-    local = max(local, (int)(rowptr[v + 1] - rowptr[v]));
-  for (int o = 16; o > 0; o >>= 1) local = max(local, __shfl_xor_sync(0xffffffffu, local, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, local);
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+    const int d = (int)(rowptr[v + 1] - rowptr[v]);
+    most = max(most, d);
+    squares += (unsigned long long)d * (unsigned)d;
+  }
+  add_degree_stats(most, squares, out);
 }
 
 std::mutex g_pool_mu;
@@ -571,13 +596,14 @@ int keys_to_csr(jgpm_graph* g, int32_t n, uint64_t* d_keys, int64_t nk, int shif
 int finish_sym(jgpm_graph* g) {
   DevBuf md(g->stream);
   int rc;
-  if ((rc = dalloc((int**)&md.p, 1, g->stream))) return rc;
-  JGPM_CUDA_TRY(cudaMemsetAsync(md.p, 0, sizeof(int), g->stream));
-  k_max_degree<<<grid_for(g->n), 256, 0, g->stream>>>(g->d_rowptr, g->n, (int*)md.p);
-  int h = 0;
-  JGPM_CUDA_TRY(cudaMemcpyAsync(&h, md.p, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  if ((rc = dalloc((DegreeStats**)&md.p, 1, g->stream))) return rc;
+  JGPM_CUDA_TRY(cudaMemsetAsync(md.p, 0, sizeof(DegreeStats), g->stream));
+  k_degree_stats<<<grid_for(g->n), 256, 0, g->stream>>>(g->d_rowptr, g->n, (DegreeStats*)md.p);
+  DegreeStats h = {0, 0};
+  JGPM_CUDA_TRY(cudaMemcpyAsync(&h, md.p, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
   JGPM_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  g->max_degree = h;
+  g->max_degree = h.most;
+  g->degree_squares = h.squares;
   return JGPM_OK;
 }
 
@@ -683,7 +709,8 @@ int upload_csr(jgpm_graph* g, const int64_t* rowptr, const int32_t* col, int32_t
   g->m = m;
   if (validate) {
     struct Check {
-      int bad, max_degree;
+      int bad;
+      DegreeStats degrees;
       unsigned long long down;
     } h;
     DevBuf st(g->stream);
@@ -691,11 +718,12 @@ int upload_csr(jgpm_graph* g, const int64_t* rowptr, const int32_t* col, int32_t
     Check* d = (Check*)st.p;
     JGPM_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(Check), g->stream));
     k_rowptr_check<<<grid_for(n), 256, 0, g->stream>>>(g->d_rowptr, n, m, &d->bad,
-                                                       &d->max_degree);
+                                                       &d->degrees);
     JGPM_CUDA_TRY(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, g->stream));
     JGPM_CUDA_TRY(cudaStreamSynchronize(g->stream));
     if (!h.bad && m > 0) {
-      g->max_degree = h.max_degree;
+      g->max_degree = h.degrees.most;
+      g->degree_squares = h.degrees.squares;
       DevBuf ob(g->stream);
       ArcOwners own;
       if ((rc = build_owners(g->d_rowptr, n, m, ob, &own))) return rc;

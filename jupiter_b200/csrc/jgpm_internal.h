@@ -92,6 +92,7 @@ struct jgpm_graph {
   int64_t* d_rowptr = nullptr;
   int32_t* d_col = nullptr;
   int32_t max_degree = 0;
+  uint64_t degree_squares = 0;  // sum of the squared degrees
   // degree-oriented DAG (built on demand)
   int64_t m_dag = 0;
   uint32_t* d_keep = nullptr;  // arc masks and counts from the validation, until the DAG is built
@@ -134,6 +135,7 @@ struct jgpm_graph {
   // statistics of the last count
   double last_kernel_ms = 0.0;
   int launches = 0;  // kernels launched since the counting call began
+  double p5_loops_us = 0.0;  // estimated time that P5 calls have spent in nested loops (plans.cu)
   int tune_min_group = 4;  // narrowest lane group for the d <= 32 roots (4, 8, 16 or 32)
   int tune_split = 128;    // roots with 32 < d <= tune_split run one per warp, above per CTA
   // timing events of the counting calls, made at the first one

@@ -25,9 +25,9 @@
 //                 induced/non-induced identities of 4-vertex graphlets.
 #include <cuda_runtime.h>
 
-#include <atomic>
-
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -832,6 +832,26 @@ int run_induced_tt(jgpm_graph* g, uint64_t* out, double* ms) {
   return JGPM_OK;
 }
 
+// Whether this P5 call uses the per-arc counters.  They need the rank DAG, which costs more than
+// the nested loops' whole count on small or sparse graphs (40,000 vertices, edge factor 4, a =
+// 0.45: a first call of 98 us in loops, 0.25 ms with counters; later ones 80 and 70 us), so the
+// first calls on such a graph run the loops, until these calls' estimated time reaches the rank
+// DAG's: whatever the number of calls, at most about twice the better of the two is spent.
+// Estimates in us, fitted to R-MAT graphs of 2,048 to 131,072 vertices, edge factors 4 to 32, a =
+// 0.45 to 0.57 (loops within a factor of two): with q the mean degree of an arc's end and x = q^2 /
+// n, which the common neighbours of an edge grow with, 0.45 + 3 sqrt(x) + 1.5 x for 1,000 edges; DAG
+// and rank DAG 175 and 0.27 for 1,000 edges.
+bool p5_by_arcs(jgpm_graph* g) {
+  if (g->d_rd_rowptr) return true;
+  const double edges = 0.5e-3 * (double)g->m;
+  const double q = g->m > 0 ? (double)g->degree_squares / (double)g->m : 0.0;
+  const double x = q * q / (double)g->n;
+  const double loops = edges * (0.45 + 3.0 * std::sqrt(x) + 1.5 * x);
+  if (g->p5_loops_us + loops >= 175.0 + 0.27 * edges) return true;
+  g->p5_loops_us += loops;
+  return false;
+}
+
 // P5 from per-arc triangle and 4-clique counters in g->d_aux (arc4.cu).
 int run_p5_arcs(jgpm_graph* g, uint64_t* out, double* ms) {
   int rc;
@@ -961,7 +981,8 @@ int count_plan_impl(jgpm_graph* g, int id, int chunk_size, unsigned flags, bool 
                     uint64_t* out, uint64_t* elements, double* ms, int* method) {
   int rc;
   const bool force_plan = (flags & JGPM_COUNT_FORCE_PLAN) != 0;
-  if (id == kP5 && !force_plan && (rc = ensure_dag(g))) return rc;
+  const bool p5_arcs = id == kP5 && !force_plan && p5_by_arcs(g);
+  if (p5_arcs && (rc = ensure_dag(g))) return rc;
   const bool force_enum = (flags & (JGPM_COUNT_FORCE_ENUM | JGPM_COUNT_FORCE_PLAN)) != 0;
   uint64_t cnt = 0;
   double t = 0.0;
@@ -971,7 +992,7 @@ int count_plan_impl(jgpm_graph* g, int id, int chunk_size, unsigned flags, bool 
   } else if (id == kP2 && !force_plan) {
     if ((rc = run_diamond_pairs(g, &cnt, &t))) return rc;
     *method = JGPM_METHOD_EDGE_TRIANGLE;
-  } else if (id == kP5 && !force_plan && arc4_fits(g)) {
+  } else if (p5_arcs && arc4_fits(g)) {
     // out-degrees up to kMidMaxDeg, where a root's symmetric bitmap fits a CTA's shared memory;
     // larger ones run the nested loops
     if ((rc = run_p5_arcs(g, &cnt, &t))) return rc;

@@ -65,3 +65,16 @@ def test_planted_cliques(gpu, sizes):
                                       (20000, 10, .45, .2391), (9000, 16, .5, .125)])
 def test_weakly_skewed(gpu, n, ef, a, b):
     check(gpu, O.rmat_graph(n, ef, a, b, b, n))
+
+
+def test_p5_after_many_calls(gpu):
+    """The nested loops of the first calls and the per-arc counters of the later ones agree."""
+    sym = O.rmat_graph(2000, 4, .5, .2, .2, 5)
+    want = O.count("P5", sym)[0]
+    with gpu.Graph.from_csr(sym.rowptr, sym.col, use_dag=False) as g:
+        methods = set()
+        for _ in range(400):
+            count, st = g.count("P5", details=True)
+            assert count == want
+            methods.add(st["method"])
+        assert len(methods) == 2
