@@ -151,15 +151,14 @@ __device__ __forceinline__ acc_t task_groups_k(const JobDesc& j, int64_t b, int6
 }
 
 template <int K, bool PAIRS, bool TT = false>
-__device__ __forceinline__ acc_t task_scan(const JobDesc& j, int64_t b, int64_t e, ScanSmem* sm) {
-  const int warp = threadIdx.x >> 5;
+__device__ __forceinline__ acc_t task_scan(const JobDesc& j, int64_t b, int64_t e, ScanSmem& sm) {
   acc_t cnt = 0, el = 0;
-  for (int64_t r = b + warp; r < e; r += 8)
-    cnt += scan_root<K, false, PAIRS, PAIRS, TT>(j.dag, j.roots[r], sm + warp, j.tri, el);
+  for (int64_t r = b; r < e; ++r)
+    cnt += scan_root<K, false, PAIRS, PAIRS, TT>(j.dag, j.roots[r], sm, j.tri, el);
   return cnt;
 }
 
-__device__ __forceinline__ acc_t task_scan_k(const JobDesc& j, int64_t b, int64_t e, ScanSmem* sm) {
+__device__ __forceinline__ acc_t task_scan_k(const JobDesc& j, int64_t b, int64_t e, ScanSmem& sm) {
   if (j.kind == kJobDiamond) return task_scan<3, true>(j, b, e, sm);
   if (j.kind == kJobIndTT) return task_scan<4, true, true>(j, b, e, sm);
   switch (j.k) {
@@ -393,7 +392,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchArgs a) {
 __global__ void __launch_bounds__(256, 4) k_batch_groups(BatchArgs a) {
   __shared__ uint32_t rows[256];
   __shared__ int degs[256];
-  __shared__ ScanSmem scans[8];
+  __shared__ ScanSmem scan;
   __shared__ unsigned long long s_task;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -410,7 +409,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_groups(BatchArgs a) {
       case kTaskGroup4: c = task_groups_k<4>(j, t.b, t.e, rows, degs); break;
       case kTaskGroup8: c = task_groups_k<8>(j, t.b, t.e, rows, degs); break;
       case kTaskGroup16: c = task_groups_k<16>(j, t.b, t.e, rows, degs); break;
-      case kTaskScanRoots: c = task_scan_k(j, t.b, t.e, scans); break;
+      case kTaskScanRoots: c = task_scan_k(j, t.b, t.e, scan); break;
       default: c = task_groups_k<32>(j, t.b, t.e, rows, degs); break;
     }
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
@@ -567,7 +566,7 @@ int build_tasks(const std::vector<BatchJobIn>& in, const jgpm_tuning& tu, BatchC
     int64_t cta_end = std::min(stop, std::max(large_end, tier_begin(t, split)));
     const int64_t warp_end = std::min(stop, std::max(cta_end, t.deg_begin[32]));
     if (t.light) {
-      add_range_tasks(light, job, kTaskScanRoots, 0, warp_end, 8);
+      add_range_tasks(light, job, kTaskScanRoots, 0, warp_end, 2);
       wide_begin = large_end = 0;
       cta_end = warp_end;
     }

@@ -23,7 +23,7 @@ enum TaskKind : int32_t {
   kTaskGroup8 = 1,
   kTaskGroup16 = 2,
   kTaskGroup32 = 3,
-  kTaskScanRoots = 12, // roots [b, e) of out-degree above 32 of a light graph, one per warp
+  kTaskScanRoots = 12, // roots [b, e) of out-degree above 32 of a light graph, the whole CTA
   kTaskWarpRoots = 4,  // roots [b, e) of out-degree 32 < d <= split, one per warp
   kTaskCtaRoot = 5,    // root b, max(split, 256) < d <= kBatchCtaMaxDeg, the whole CTA, masks
                        // of up to 16 words in registers

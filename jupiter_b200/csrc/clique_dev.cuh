@@ -635,52 +635,49 @@ __device__ __forceinline__ int row_members(const uint32_t* Ri, int w_d, uint16_t
   return c;
 }
 
-// One root of out-degree d <= kLightOutDegree of a graph without a rank DAG, on one warp: its rows
-// are scanned four at a time and looked up in the list in shared memory.
+// One root of out-degree d <= kLightOutDegree of a graph without a rank DAG, on a CTA of 256
+// threads: the warps scan the rows, four at a time, and look their elements up in the list in shared
+// memory.  Such roots are few, so what counts is how long one takes.
 struct ScanSmem {
+  eid_t s[kLightOutDegree];
+  int len[kLightOutDegree];
   int L[kLightOutDegree];
-  int deg[kLightOutDegree];  // out-degrees (accounting) or hits per list entry (ETRI)
+  int hits[kLightOutDegree];  // per list entry (ETRI)
   uint32_t R[kLightOutDegree * 2];
 };
 template <int K, bool STATS, bool ETRI, bool PAIRS = false, bool TT = false>
-__device__ __forceinline__ acc_t scan_root(const RankDag& g, vid_t u, ScanSmem* sm, uint32_t* tri,
+__device__ __forceinline__ acc_t scan_root(const RankDag& g, vid_t u, ScanSmem& sm, uint32_t* tri,
                                            acc_t& elems) {
-  static_assert(kLightOutDegree == 64, "two list entries and two row elements a lane");
+  static_assert(kLightOutDegree == 64, "two row elements a lane, four threads a row");
   constexpr int U = 4;
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const eid_t base = g.rp[u];
   const int d = (int)(g.rp[u + 1] - base);
-  vid_t L[2];
-  eid_t s[2];
-  int len[2];
-  __syncwarp();  // the last root's readers are done
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const int j = 32 * b + lane;
-    L[b] = j < d ? __ldg(g.col + base + j) : INT32_MAX;
-    s[b] = j < d ? g.rp[L[b]] : 0;
-    len[b] = j < d ? (int)(g.rp[L[b] + 1] - s[b]) : 0;
-    sm->L[j] = L[b];
-    sm->deg[j] = STATS ? len[b] : 0;
-    sm->R[2 * j] = sm->R[2 * j + 1] = 0u;
+  __syncthreads();  // the last root's readers are done
+  if (tid < kLightOutDegree) {
+    const vid_t x = tid < d ? __ldg(g.col + base + tid) : INT32_MAX;
+    const eid_t s = tid < d ? g.rp[x] : 0;
+    sm.L[tid] = x;
+    sm.s[tid] = s;
+    sm.len[tid] = tid < d ? (int)(g.rp[x + 1] - s) : 0;
+    sm.hits[tid] = 0;
+    sm.R[2 * tid] = sm.R[2 * tid + 1] = 0u;
   }
-  __syncwarp();
+  __syncthreads();
   acc_t cnt = 0, pairs = 0, tt = 0;
-  for (int i0 = 0; i0 < d; i0 += U) {
+  for (int i0 = warp; i0 < d; i0 += 8 * U) {
     eid_t e[U][2];
     vid_t x[U][2];
+    unsigned old[U][2];
 #pragma unroll
     for (int t = 0; t < U; ++t) {
-      const int i = i0 + t;
-      const int ln = i < d ? __shfl_sync(kFull, i < 32 ? len[0] : len[1], i & 31) : 0;
-      const eid_t si = __shfl_sync(kFull, i < 32 ? s[0] : s[1], i & 31);
+      const int i = min(i0 + 8 * t, kLightOutDegree - 1), ln = i0 + 8 * t < d ? sm.len[i] : 0;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        e[t][h] = si + 32 * h + lane;
+        e[t][h] = sm.s[i] + 32 * h + lane;
         x[t][h] = 32 * h + lane < ln ? __ldg(g.col + e[t][h]) : -1;
       }
     }
-    unsigned old[U][2];
 #pragma unroll
     for (int t = 0; t < U; ++t) {
 #pragma unroll
@@ -689,14 +686,14 @@ __device__ __forceinline__ acc_t scan_root(const RankDag& g, vid_t u, ScanSmem* 
         int p = 0;
 #pragma unroll
         for (int step = 32; step > 0; step >>= 1)
-          if (sm->L[p + step - 1] < x[t][h]) p += step;
-        if (x[t][h] < 0 || sm->L[p] != x[t][h]) continue;
+          if (sm.L[p + step - 1] < x[t][h]) p += step;
+        if (x[t][h] < 0 || sm.L[p] != x[t][h]) continue;
         if (ETRI) {
           old[t][h] = atomicAdd(tri + e[t][h], 1u);
-          atomicAdd(&sm->deg[p], 1);
+          atomicAdd(&sm.hits[p], 1);
         }
         if (K == 3) ++cnt;
-        atomicOr(&sm->R[2 * (i0 + t) + (p >> 5)], 1u << (p & 31));
+        atomicOr(&sm.R[2 * (i0 + 8 * t) + (p >> 5)], 1u << (p & 31));
       }
     }
     if (PAIRS) {
@@ -704,26 +701,32 @@ __device__ __forceinline__ acc_t scan_root(const RankDag& g, vid_t u, ScanSmem* 
       for (int t = 0; t < U; ++t) pairs += (acc_t)old[t][0] + (acc_t)old[t][1];
     }
   }
-  __syncwarp();
-  if (K > 3) {
-    for (int i = lane; i < d; i += 32) {
-      const uint32_t m[2] = {sm->R[2 * i], sm->R[2 * i + 1]};
-      cnt += RowCount<(K > 3 ? K - 3 : 1), 2, STATS>::run(m, sm->R, 2, sm->deg, elems, 2);
+  __syncthreads();
+  const int i = tid >> 2;
+  if (K > 3 && i < d) {  // four threads take the members of row i in turn
+    const uint32_t m[2] = {sm.R[2 * i], sm.R[2 * i + 1]};
+    const int pm = __popc(m[0]) + __popc(m[1]);
+    int at = tid & 3;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      for (uint32_t w = m[q]; w != 0u; w &= w - 1u, ++at) {
+        if ((at & 3) != 0) continue;
+        const int j = 32 * q + __ffs(w) - 1;
+        if (STATS) elems += (acc_t)pm + (acc_t)sm.len[j];
+        const uint32_t nxt[2] = {m[0] & sm.R[2 * j], m[1] & sm.R[2 * j + 1]};
+        cnt += RowCount<(K > 3 ? K - 4 : 0), 2, STATS>::run(nxt, sm.R, 2, sm.len, elems, 2);
+      }
     }
   }
-  if (ETRI) {  // the root's own arcs, as in group_root
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = 32 * b + lane;
-      const unsigned rowc = (unsigned)(__popc(sm->R[2 * i]) + __popc(sm->R[2 * i + 1]));
-      const unsigned colc = (unsigned)sm->deg[i], tu = rowc + colc;
-      if (i < d && tu) {
-        const unsigned o = atomicAdd(tri + base + i, tu);
-        if (PAIRS) pairs += pair_gain(o, tu);
-        if (TT) {
-          const acc_t di = tt_deg(g, L[b]);
-          tt += (acc_t)rowc * (tt_deg(g, u) + di) + (acc_t)colc * di;
-        }
+  if (ETRI && tid < d) {  // the root's own arcs, as in group_root
+    const unsigned rowc = (unsigned)(__popc(sm.R[2 * tid]) + __popc(sm.R[2 * tid + 1]));
+    const unsigned colc = (unsigned)sm.hits[tid], tu = rowc + colc;
+    if (tu) {
+      const unsigned o = atomicAdd(tri + base + tid, tu);
+      if (PAIRS) pairs += pair_gain(o, tu);
+      if (TT) {
+        const acc_t di = tt_deg(g, sm.L[tid]);
+        tt += (acc_t)rowc * (tt_deg(g, u) + di) + (acc_t)colc * di;
       }
     }
   }

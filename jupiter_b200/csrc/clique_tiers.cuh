@@ -185,21 +185,14 @@ __global__ void __launch_bounds__(256, 4) k_clique_warp(CliqueArgs a) {
   pdl_close();
 }
 
-// --------------------------------- roots above 32 of a graph without a rank DAG, one per warp
+// ------------------------------------------- roots above 32 of a graph without a rank DAG
 template <int K, bool STATS, bool ETRI = false, bool PAIRS = false, bool TT = false>
 __global__ void __launch_bounds__(256) k_clique_scan(CliqueArgs a) {
-  __shared__ ScanSmem sm[8];
-  const int lane = threadIdx.x & 31;
+  __shared__ ScanSmem sm;
   pdl_open();
   acc_t cnt = 0, elems = 0;
-  for (;;) {
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(&a.ctl->counter[a.cursor], 1ull);
-    const int64_t idx = a.begin + (int64_t)__shfl_sync(kFull, c, 0);
-    if (idx >= a.end) break;
-    cnt += scan_root<K, STATS, ETRI, PAIRS, TT>(a.dag, root_at(a, idx), &sm[threadIdx.x >> 5],
-                                                a.tri, elems);
-  }
+  for (int64_t i = a.begin + blockIdx.x; i < a.end; i += gridDim.x)
+    cnt += scan_root<K, STATS, ETRI, PAIRS, TT>(a.dag, root_at(a, i), sm, a.tri, elems);
   add_result<STATS>(a.ctl, cnt, elems);
   pdl_close();
 }
@@ -462,8 +455,7 @@ int launch_plan_k(const CliqueArgs& base, const TierPlan& p, int sms, cudaStream
     a.begin = p.scan.b;
     a.end = p.scan.e;
     a.step = p.scan.step;
-    a.cursor = 7;
-    const int64_t grid = std::min<int64_t>((int64_t)sms * 4, (a.end - a.begin + 7) / 8);
+    const int64_t grid = std::min<int64_t>((int64_t)sms * 4, a.end - a.begin);
     const cudaError_t rc =
         tier_launch(pdl(), k_clique_scan<K, STATS, ETRI, PAIRS, TT>, (int)grid, 0, s, a);
     ++n;
@@ -480,7 +472,10 @@ int launch_plan_k(const CliqueArgs& base, const TierPlan& p, int sms, cudaStream
     auto kern = k_clique_small<K, STATS, ETRI, PAIRS, TT>;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
-    const int64_t grid = std::min<int64_t>((int64_t)sms * std::max(1, per_sm), (tasks + 7) / 8);
+    // behind other tiers, whose last CTAs it overlaps, it leaves them room: five CTAs (triangles of
+    // 65,536 vertices, edge factor 16: 83 us, 88 with eight)
+    per_sm = std::max(1, n > 0 ? std::min(per_sm, 5) : per_sm);
+    const int64_t grid = std::min<int64_t>((int64_t)sms * per_sm, (tasks + 7) / 8);
     const cudaError_t rc = tier_launch(pdl(), kern, (int)grid, 0, s, a, sr);
     ++n;
     if (launch_failed(&err, rc)) return -1;

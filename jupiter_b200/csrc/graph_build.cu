@@ -1335,10 +1335,13 @@ int ensure_rank_dag(jgpm_graph* g) {
 // DAG and id DAG: 4-cliques of 40,000 vertices, edge factor 8, a = 0.51: 165 and 122 | 54 and 53; of
 // 4,194,304 vertices, edge factor 4, a = 0.51 (out-degrees up to 44): 1,186 and 767 | 574 and 620.
 // A graph that lies in the bitmap whole, with some 12 arcs a vertex or more, is better off there
-// (2,500 vertices, edge factor 32, a = 0.45: 116 and 88 | 40 and 49), and so are graphs with more
-// roots above 32 entries, whose pairs grow with the square.
+// (2,500 vertices, edge factor 32, a = 0.45: 116 and 88 | 40 and 49), and so are graphs with many
+// roots above 32 entries, whose pairs grow with the square, or of less than 4 M arcs with a few of
+// them, which cost a launch more (8,273 vertices, edge factor 16, a = 0.451: 160 and 127 | 44 and
+// 59).
 bool light_dag(const jgpm_graph* g) {
-  if (g->max_out_degree > kLightOutDegree || g->over32 > g->m_dag / 2048) return false;
+  if (g->max_out_degree > kLightOutDegree) return false;
+  if (g->over32 > 0) return g->m_dag >= (int64_t)1 << 22 && g->over32 <= g->m_dag / 2048;
   return g->m_dag < 12 * (int64_t)g->n || rank_top(g->n, g->m_dag) < g->n;
 }
 

@@ -446,12 +446,13 @@ int jgpm_setop_batch(int op, const int32_t* a, const int64_t* a_off, const int32
       mat ? off.out.d : nullptr, off.check);
   cudaError_t e = cudaGetLastError();
   // a refused call writes nothing: the staged results are copied back once the verdict is read
+  const bool waits = !off.checked;  // for the kernel, to read the verdict
   if (e == cudaSuccess && (rc = off.verdict("jgpm_setop_batch"))) return rc;
   if (e == cudaSuccess && counts_host)
     e = cudaMemcpyAsync(counts, dcounts, nops * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && out_host && off.out_end > 0)
     e = cudaMemcpyAsync(out, dout, off.out_end * 4, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && (!waits || counts_host || out_host)) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     jgpm_set_error_(std::string("jgpm_setop_batch: ") + cudaGetErrorString(e));
     return JGPM_ECUDA;

@@ -152,8 +152,10 @@ __device__ __forceinline__ void warp_lookup(const int32_t* a, int na, const int3
   }
   if (base < na) {
     const int i = base + lane;
-    const int32_t key = i < na ? __ldg(a + i) : INT32_MAX;
-    visit(key, i < na, i < na && contains_g(b, nb, key));
+    int32_t key[1] = {i < na ? __ldg(a + i) : INT32_MAX};
+    bool hit[1];
+    contains_u<1>(b, nb, key, hit);
+    visit(key[0], i < na, hit[0]);
   }
 }
 
