@@ -198,7 +198,7 @@ __device__ __forceinline__ void scan_rows(const RankDag& g, vid_t Lj, int d, eid
 // one count per triangle arc.
 //
 // Rows of the graph's top h vertices are tested pair by pair in the bitmap, four rows at a time so
-// that their loads overlap.  The other rows, which are short, are scanned (scan_rows): their
+// that their loads overlap (eight in a triangle count, which keeps nothing of them).  The other rows, which are short, are scanned (scan_rows): their
 // elements are read once, in order, where a binary search per pair is a chain of scattered loads
 // (R-MAT, 1,048,576 vertices, edge factor 16, a = 0.45, 84 % of the pairs outside the bitmap: a
 // triangle count of 1.79 ms with searches, 0.80 ms with scans; kScanAhead = 1: 0.85 ms).
@@ -206,7 +206,7 @@ template <int G, int K, bool STATS, bool ETRI, bool PAIRS = false, bool TT = fal
 __device__ __forceinline__ acc_t group_root(const RankDag& g, vid_t u, uint32_t* R, int* DG,
                                             uint32_t* tri, acc_t& elems) {
   constexpr bool STORE = K >= 5 || STATS;
-  constexpr int U = 4;
+  constexpr int U = K == 3 && !ETRI && !STATS && G >= 8 ? 8 : 4;
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);
   const int gsh = lane & ~(G - 1);

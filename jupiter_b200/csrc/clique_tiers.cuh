@@ -472,9 +472,11 @@ int launch_plan_k(const CliqueArgs& base, const TierPlan& p, int sms, cudaStream
     auto kern = k_clique_small<K, STATS, ETRI, PAIRS, TT>;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
-    // behind other tiers, whose last CTAs it overlaps, it leaves them room: five CTAs (triangles of
-    // 65,536 vertices, edge factor 16: 83 us, 88 with eight)
-    per_sm = std::max(1, n > 0 ? std::min(per_sm, 5) : per_sm);
+    // a short launch behind other tiers, whose last CTAs it overlaps, leaves them room: five CTAs
+    // per SM (triangles of 65,536 vertices, edge factor 16: 85 us, 88 with as many as fit; a long
+    // one, of 4,194,304 vertices, edge factor 4, a = 0.45, b = 0.2391: 0.81 and 0.71 ms)
+    if (n > 0 && tasks < (int64_t)sms * 1024) per_sm = std::min(per_sm, 5);
+    per_sm = std::max(1, per_sm);
     const int64_t grid = std::min<int64_t>((int64_t)sms * per_sm, (tasks + 7) / 8);
     const cudaError_t rc = tier_launch(pdl(), kern, (int)grid, 0, s, a, sr);
     ++n;
