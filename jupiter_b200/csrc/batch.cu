@@ -73,15 +73,15 @@ constexpr int kLevels = 6;
 // buffers fit the shared memory that the other task kinds need anyway (34 KB).  Above 256 they
 // would halve the CTAs per SM, so those roots flatten their (row, bit) pairs.
 constexpr int kBatchK5Deg = 256, kBatchK5Words = kBatchK5Deg / 32;
-constexpr MidLayout kBatchK5Layout{kBatchK5Deg, kBatchK5Words, kBatchK5Words};
+constexpr MidLayout kBatchK5Layout{kBatchK5Deg, row_words<5>(kBatchK5Words), kBatchK5Words};
 
 // Shared memory of one CTA of the batched kernel: the largest of the per-kind layouts.
 inline size_t batch_smem_bytes(int dmax, int W, int wdmax, int wW) {
   size_t b = std::max(8 * sizeof(WarpSmem), kBatchK5Layout.bytes());
   b = std::max(b, 8 * sizeof(C4WarpHash));
   b = std::max(b, sizeof(C4MidSmem<256>));
-  b = std::max(b, MidLayout{dmax, W}.bytes());
-  if (wdmax > 0) b = std::max(b, MidLayout{wdmax, wW}.bytes_no_rows());
+  b = std::max(b, MidLayout{dmax, row_words<0>(W)}.bytes());
+  if (wdmax > 0) b = std::max(b, MidLayout{wdmax, 0}.bytes_no_rows());
   return b;
 }
 
@@ -208,24 +208,29 @@ __device__ __forceinline__ acc_t task_warp_roots(const JobDesc& j, int64_t b, in
 template <int K, int W>
 constexpr int batch_row_words() { return K >= 7 || (K >= 6 && W > 8) ? 0 : W; }
 
-// One CTA root with rows of up to W words (out-degree <= 32 W), masks in registers.
+// One CTA root of a count that works on tiles (k <= 4, diamonds, tailed triangles).
+__device__ __forceinline__ acc_t task_cta_tiles(const JobDesc& j, vid_t u, const MidSmem& sm) {
+  acc_t el = 0;
+  if (j.kind == kJobDiamond) return cta_root<3, false, true, true, 0>(j.dag, u, sm, j.tri, el);
+  if (j.kind == kJobIndTT)
+    return cta_root<4, false, true, true, 0, 1, false, true>(j.dag, u, sm, j.tri, el);
+  if (j.k == 3) return cta_root<3, false, false, false, 0>(j.dag, u, sm, nullptr, el);
+  return cta_root<4, false, false, false, 0>(j.dag, u, sm, nullptr, el);
+}
+
+// One CTA root of k >= 5 with rows of up to W words (out-degree <= 32 W), masks in registers.
 // sm5: the layout of the 5-clique count (kBatchK5Layout).
 template <int W>
 __device__ __forceinline__ acc_t task_cta_root(const JobDesc& j, vid_t u, const MidSmem& sm,
                                                const MidSmem& sm5) {
   acc_t el = 0;
-  if (j.kind == kJobDiamond)  // pair mode returns before the mask counting
-    return cta_root<3, false, true, true, 0>(j.dag, u, sm, j.tri, el);
-  if (j.kind == kJobIndTT)
-    return cta_root<4, false, true, true, W, 1, false, true>(j.dag, u, sm, j.tri, el);
   switch (j.k) {
-    case 3: return cta_root<3, false, false, false, W>(j.dag, u, sm, nullptr, el);
-    case 4: return cta_root<4, false, false, false, W>(j.dag, u, sm, nullptr, el);
     case 5:
-      if (W == kBatchK5Words)
-        return cta_root<5, false, false, false, kBatchK5Words, 1, false, false, true>(
-            j.dag, u, sm5, nullptr, el);
-      return cta_root<5, false, false, false, W>(j.dag, u, sm, nullptr, el);
+      if constexpr (W == kBatchK5Words)
+        return cta_root<5, false, false, false, W, 1, false, false, true>(j.dag, u, sm5, nullptr,
+                                                                          el);
+      else
+        return cta_root<5, false, false, false, W>(j.dag, u, sm, nullptr, el);
     case 6:
       return cta_root<6, false, false, false, batch_row_words<6, W>()>(j.dag, u, sm,
                                                                        nullptr, el);
@@ -323,9 +328,9 @@ __device__ __forceinline__ acc_t task_c4_small(const JobDesc& j, int64_t b, int6
 
 __global__ void __launch_bounds__(256, 4) k_batch(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const MidSmem sm = MidSmem::carve(smem, a.dmax, a.W);
+  const MidSmem sm = MidSmem::carve(smem, a.dmax, row_words<0>(a.W));
   const MidSmem sm5 =
-      MidSmem::carve(smem, kBatchK5Deg, kBatchK5Words, nullptr, kBatchK5Words);
+      MidSmem::carve(smem, kBatchK5Deg, kBatchK5Layout.row_w, nullptr, kBatchK5Words);
   WarpSmem& ws = reinterpret_cast<WarpSmem*>(smem)[threadIdx.x >> 5];
   C4WarpHash& hash = reinterpret_cast<C4WarpHash*>(smem)[threadIdx.x >> 5];
   C4MidSmem<256>& c4m = *reinterpret_cast<C4MidSmem<256>*>(smem);
@@ -351,12 +356,11 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchArgs a) {
         c = task_warp_roots(j, t.b, t.e, ws, &s_next);
         break;
       case kTaskCtaRoot:
-        smem_kind = kTaskCtaRoot;
-        c = task_cta_root<16>(j, j.roots[t.b], sm, sm5);
-        break;
       case kTaskCtaRoot8:
         smem_kind = kTaskCtaRoot;
-        c = task_cta_root<8>(j, j.roots[t.b], sm, sm5);
+        c = j.k <= 4                 ? task_cta_tiles(j, j.roots[t.b], sm)
+            : t.kind == kTaskCtaRoot ? task_cta_root<16>(j, j.roots[t.b], sm, sm5)
+                                     : task_cta_root<8>(j, j.roots[t.b], sm, sm5);
         break;
       case kTaskWideRoot: {
         smem_kind = kTaskWideRoot;

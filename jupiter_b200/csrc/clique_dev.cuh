@@ -49,17 +49,12 @@ __device__ __forceinline__ acc_t pair_gain(unsigned o, unsigned k) {
 // Largest power of two <= n (0 for n <= 0).
 __device__ __forceinline__ int top_pow2(int n) { return n > 0 ? 1 << (31 - __clz(n)) : 0; }
 
-// Two independent searches in the same sorted shared-memory array a[0..n) in lockstep:
-// p0 = #{a[j] < x0}, p1 = #{a[j] < x1}.  Binary lifting with a fixed trip count (top =
-// top_pow2(n)), so the two dependent load chains overlap.
-__device__ __forceinline__ void count_below2(const int* a, int n, int top, int x0, int x1,
-                                             int& p0, int& p1) {
-  p0 = 0;
-  p1 = 0;
-  for (int step = top; step > 0; step >>= 1) {
-    if (p0 + step <= n && a[p0 + step - 1] < x0) p0 += step;
-    if (p1 + step <= n && a[p1 + step - 1] < x1) p1 += step;
-  }
+// Elements of the sorted shared-memory array a[0..n) below x, by binary lifting (top = top_pow2(n)).
+__device__ __forceinline__ int count_below(const int* a, int n, int top, int x) {
+  int p = 0;
+  for (int step = top; step > 0; step >>= 1)
+    if (p + step <= n && a[p + step - 1] < x) p += step;
+  return p;
 }
 
 // Symmetric degree minus two (the tailed-triangle degree term of a triangle vertex).
@@ -936,8 +931,7 @@ __device__ __forceinline__ acc_t warp_root(const RankDag& g, vid_t u, WarpSmem* 
       __syncwarp();
       const int P = off[d], topO = top_pow2(d - 1);
       for (int p = lane; p < P; p += 32) {
-        int i, i2;
-        count_below2(off + 1, d - 1, topO, p + 1, p + 1, i, i2);
+        const int i = count_below(off + 1, d - 1, topO, p + 1);
         const uint32_t* Ri = R + i * w_d;
         const int j = select_bit(Ri, w_d, p - off[i]);
         const uint32_t* Rj = R + j * w_d;
@@ -989,10 +983,14 @@ __host__ __device__ __forceinline__ int row_stride(int w_d, bool global_rows) {
   if (global_rows) return w_d;
   return K == 4 ? (((w_d + 3) >> 2) | 1) << 2 : (w_d | 1);
 }
-// The largest of them: what a layout for any k allots per row.
-__host__ __device__ __forceinline__ int row_words(int w_d) {
-  const int odd = w_d | 1, four = row_stride<4>(w_d, false);
-  return odd > four ? odd : four;
+// Words that a layout allots per row of up to W words: none for the triangle counts, which keep no
+// rows (K = 3 without accounting), else the most that any k takes.  (The 5-clique bands are the
+// slower with only their own: one CTA more per SM takes L1 from the pair tests; 65,536 vertices,
+// edge factor 16: 0.96 ms, 1.36 ms so.)
+template <int K, bool STATS = false>
+__host__ __device__ constexpr int row_words(int W) {
+  const int odd = W | 1, four = (((W + 3) >> 2) | 1) << 2;
+  return K == 3 && !STATS ? 0 : odd > four ? odd : four;
 }
 
 // Balanced 5-clique count of the widest band (BAL, rows of up to 32 words): per warp, the
@@ -1023,13 +1021,13 @@ __host__ __device__ __forceinline__ size_t k5_bytes(int rw, int dmax) {
 
 // Shared layout for one mid-tier root (dynamic shared memory):
 //   L[dmax] ids | rb[dmax] bitmap rows | off[dmax+1] pair offsets, or row counts | deg[dmax]
-//   out-degrees, or column counts | R[dmax * row_words(W)] rows | 8 warp sums | 5-clique buffers
-//   (bal_rw)
+//   out-degrees, or column counts | R[dmax * row_w] rows | 8 warp sums | 5-clique buffers (bal_rw)
 struct MidLayout {
-  int dmax, W;
+  int dmax;
+  int row_w;       // words allotted per row (row_words)
   int bal_rw = 0;  // mask words of the 5-clique buffers (0: none)
   __host__ __device__ size_t bytes() const {
-    return bytes_no_rows() + (size_t)dmax * row_words(W) * 4;
+    return bytes_no_rows() + (size_t)dmax * row_w * 4;
   }
   __host__ __device__ size_t bytes_no_rows() const {
     return (size_t)dmax * 16 + 4 + 16 + 64 + 64 + k5_bytes(bal_rw, dmax);
@@ -1053,7 +1051,7 @@ struct MidSmem {
   // rows = nullptr: the rows follow in shared memory (MidLayout); otherwise they live at
   // rows (dmax * W words of global scratch for this CTA) and shared memory holds the rest
   // (MidLayout::bytes_no_rows).
-  __device__ __forceinline__ static MidSmem carve(unsigned char* smem, int dmax, int W,
+  __device__ __forceinline__ static MidSmem carve(unsigned char* smem, int dmax, int row_w,
                                                   uint32_t* rows = nullptr, int bal_rw = 0) {
     MidSmem m;
     m.L = reinterpret_cast<vid_t*>(smem);
@@ -1068,7 +1066,7 @@ struct MidSmem {
       m.wsum = reinterpret_cast<int*>(after);
     } else {
       m.R = after;
-      m.wsum = reinterpret_cast<int*>(m.R + (size_t)dmax * row_words(W));
+      m.wsum = reinterpret_cast<int*>(m.R + (size_t)dmax * row_w);
     }
     m.k5_next = reinterpret_cast<int*>(
         (reinterpret_cast<uintptr_t>(m.wsum + 8) + 15) & ~uintptr_t(15));
@@ -1133,18 +1131,14 @@ __device__ __forceinline__ acc_t bal_items_w(const uint16_t* Lw, int nit, const 
   return cnt;
 }
 
-template <int RW>
+// Rows of 17 to 32 words (the band of out-degree 513 to 1,024).
 __device__ __forceinline__ acc_t bal_items(const uint16_t* Lw, int nit, const uint32_t* Mw,
                                            const uint32_t* R, int S, int w_d) {
   switch ((w_d + 3) >> 2) {
-    case 1: return bal_items_w<4>(Lw, nit, Mw, R, S);
-    case 2: return bal_items_w<(RW >= 8 ? 8 : 4)>(Lw, nit, Mw, R, S);
-    case 3: return bal_items_w<(RW >= 12 ? 12 : 4)>(Lw, nit, Mw, R, S);
-    case 4: return bal_items_w<(RW >= 16 ? 16 : 4)>(Lw, nit, Mw, R, S);
-    case 5: return bal_items_w<(RW >= 20 ? 20 : 4)>(Lw, nit, Mw, R, S);
-    case 6: return bal_items_w<(RW >= 24 ? 24 : 4)>(Lw, nit, Mw, R, S);
-    case 7: return bal_items_w<(RW >= 28 ? 28 : 4)>(Lw, nit, Mw, R, S);
-    default: return bal_items_w<(RW >= 32 ? 32 : 4)>(Lw, nit, Mw, R, S);
+    case 5: return bal_items_w<20>(Lw, nit, Mw, R, S);
+    case 6: return bal_items_w<24>(Lw, nit, Mw, R, S);
+    case 7: return bal_items_w<28>(Lw, nit, Mw, R, S);
+    default: return bal_items_w<32>(Lw, nit, Mw, R, S);
   }
 }
 
@@ -1168,8 +1162,7 @@ __device__ __forceinline__ acc_t bal_count5(const int* off, int d, int topO,
     uint32_t m2[RW];
     int c = 0;
     if (p < P) {
-      int i, i2;
-      count_below2(off + 1, d - 1, topO, p + 1, p + 1, i, i2);
+      const int i = count_below(off + 1, d - 1, topO, p + 1);
       const uint32_t* Ri = R + (size_t)i * S;
       const int j = select_bit(Ri, w_d, p - off[i]);
       const uint32_t* Rj = R + (size_t)j * S;
@@ -1216,7 +1209,7 @@ __device__ __forceinline__ acc_t bal_count5(const int* off, int d, int topO,
       }
       __syncwarp();
       const int nit = min(C - r0, kBalCap);
-      cnt += bal_items<RW>(Lw, nit, Mw, R, S, w_d);
+      cnt += bal_items(Lw, nit, Mw, R, S, w_d);
       __syncwarp();
     }
   }
@@ -1446,8 +1439,7 @@ __device__ __forceinline__ acc_t cta_root(const RankDag& g, vid_t u, const MidSm
     } else {
       const int P = off[d];
       for (int p = tid; p < P; p += nthreads) {
-        int i, i2;
-        count_below2(off + 1, d - 1, topO, p + 1, p + 1, i, i2);
+        const int i = count_below(off + 1, d - 1, topO, p + 1);
         const uint32_t* Ri = R + (size_t)i * S;
         const int j = select_bit(Ri, w_d, p - off[i]);
         const uint32_t* Rj = R + (size_t)j * S;

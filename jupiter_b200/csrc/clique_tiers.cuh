@@ -212,7 +212,7 @@ template <int K, bool STATS, bool ETRI = false, bool PAIRS = false, int ROWW = k
 __global__ void __launch_bounds__(256, kMidMinBlocks<K, STATS, BAL, ROWW>())
     k_clique_mid(CliqueArgs a, int dmax, int W) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const MidSmem sm = MidSmem::carve(smem, dmax, W,
+  const MidSmem sm = MidSmem::carve(smem, dmax, row_words<K, STATS>(W),
                                     GR ? a.rows + (size_t)blockIdx.x * dmax * W : nullptr,
                                     BAL ? ROWW : 0);
   __shared__ unsigned long long s_idx[2];
@@ -348,16 +348,16 @@ cudaError_t tier_launch(bool pdl, void (*kern)(Args...), int grid, size_t smem, 
   return launch_pdl(pdl, kern, grid, 256, smem, s, args...);
 }
 
-// Register-mask width of a CTA band: k >= 7 counts warp-cooperatively (0), which keeps the
-// deep register-mask recursion, and its compile time, out of the large clique sizes.
-template <int K>
-constexpr int kBandRowWords(int w) { return K >= 7 ? 0 : w; }
+// Mask words that a CTA band counts from registers.  None (0) where nothing is: the plain counts of
+// k <= 4, which work on tiles (one kernel for all bands), and k >= 7, counted warp-cooperatively,
+// which keeps the deep register-mask recursion, and its compile time, out of the large sizes.
+template <int K, bool STATS>
+constexpr int kBandRowWords(int w) { return K >= 7 || (K <= 4 && !STATS) ? 0 : w; }
 
-// Mask words counted from registers in the band of out-degree <= 1024 (rows of up to 32
-// words): k = 4 row-parallel, k = 5 over (row, bit) pairs, one 32-word mask per thread; the
-// warp-cooperative form (0) otherwise.
-template <int K>
-constexpr int kWideBandRowWords() { return K == 4 || K == 5 ? 32 : 0; }
+// The same for the band of out-degree <= 1024 (rows of up to 32 words): k = 5 over (row, bit) pairs
+// and the accounting of k = 4 row-parallel, one 32-word mask per thread.
+template <int K, bool STATS>
+constexpr int kWideBandRowWords() { return (K == 4 && STATS) || K == 5 ? 32 : 0; }
 
 // One CTA-root band: bitmap layout for out-degree <= dmax, masks of up to ROWW words counted
 // from registers, wider ones with WPL words per lane; GR puts the rows in global scratch.
@@ -375,7 +375,7 @@ cudaError_t launch_mid_band(CliqueArgs a, const TierRange& r, int cursor, int dm
   a.cursor = cursor;
   const int W = (dmax + 31) / 32;
   constexpr bool BAL = kBandBalanced<K, STATS, ETRI, ROWW, GR>();
-  const MidLayout lay{dmax, W, BAL ? ROWW : 0};
+  const MidLayout lay{dmax, row_words<K, STATS>(W), BAL ? ROWW : 0};
   const size_t sm = GR ? lay.bytes_no_rows() : lay.bytes();
   auto kern = k_clique_mid<K, STATS, ETRI, PAIRS, ROWW, WPL, GR, TT, BAL>;
   raise_smem_limit((const void*)kern, sm);  // a failure shows up as the launch error
@@ -415,21 +415,21 @@ int launch_plan_k(const CliqueArgs& base, const TierPlan& p, int sms, cudaStream
   }
   if (!p.mid[0].empty()) {
     const cudaError_t rc =
-        launch_mid_band<K, STATS, ETRI, PAIRS, kWideBandRowWords<K>(), 1, false, TT>(
+        launch_mid_band<K, STATS, ETRI, PAIRS, kWideBandRowWords<K, STATS>(), 1, false, TT>(
             a, p.mid[0], 1, std::min(max_out, kMidMaxDeg), sms, s, pdl());
     ++n;
     if (launch_failed(&err, rc)) return -1;
   }
   if (!p.mid[1].empty()) {
     const cudaError_t rc =
-        launch_mid_band<K, STATS, ETRI, PAIRS, kBandRowWords<K>(16), 1, false, TT>(
+        launch_mid_band<K, STATS, ETRI, PAIRS, kBandRowWords<K, STATS>(16), 1, false, TT>(
             a, p.mid[1], 0, std::min(max_out, 512), sms, s, pdl());
     ++n;
     if (launch_failed(&err, rc)) return -1;
   }
   if (!p.mid[2].empty()) {
     const cudaError_t rc =
-        launch_mid_band<K, STATS, ETRI, PAIRS, kBandRowWords<K>(8), 1, false, TT>(
+        launch_mid_band<K, STATS, ETRI, PAIRS, kBandRowWords<K, STATS>(8), 1, false, TT>(
             a, p.mid[2], 8, std::min(max_out, 256), sms, s, pdl());
     ++n;
     if (launch_failed(&err, rc)) return -1;
