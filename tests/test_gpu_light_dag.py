@@ -1,7 +1,8 @@
-"""Graphs that are counted on the id DAG, by scans (small out-degrees, few vertices above 32), and
-the borders of that rule: planted complete graphs bring roots of out-degree 32, 33, 63, 64 and 65
-(the last is past it) into a sparse graph; weakly skewed R-MAT graphs have short rows outside the
-bitmap.  Counts are integers: equality with the oracle, single calls, batches and shards."""
+"""Graphs that are counted on the id DAG, by scans (out-degrees up to 32; on graphs of 4 M arcs and
+more up to 64, with few vertices above 32), and the borders of that rule: planted complete graphs
+bring roots of out-degree 32, 33, 63, 64 and 65 into sparse graphs; weakly skewed R-MAT graphs have
+short rows outside the bitmap.  Counts are integers: equality with the oracle, single calls,
+batches and shards."""
 import numpy as np
 import pytest
 
@@ -34,7 +35,7 @@ def wanted(sym):
     return want, O.count("induced-tailed-triangle", sym)[0], dag
 
 
-def check(gpu, sym):
+def check(gpu, sym, p5=True):
     want, tt, dag = wanted(sym)
     with gpu.Graph.from_csr(sym.rowptr, sym.col, use_dag=False) as g:
         for k, w in want.items():
@@ -49,15 +50,22 @@ def check(gpu, sym):
         got = gpu.batch_count(jobs)[0]
         assert got[:-1] == list(want.values()) + [tt]
         assert got[-1] == g.count("k-clique:7")
-        # P5 may move the graph to the rank DAG; the counts stay
-        p5 = O.count("P5", sym)[0]
-        assert [g.count("P5") for _ in range(3)] == [p5] * 3
+        if p5:  # may move the graph to the rank DAG; the counts stay
+            p5 = O.count("P5", sym)[0]
+            assert [g.count("P5") for _ in range(3)] == [p5] * 3
         assert g.count("triangle") == want["triangle"]
 
 
 @pytest.mark.parametrize("sizes", [(), (33,), (34,), (33, 34, 40), (64,), (65,), (66,), (20,) * 40])
 def test_planted_cliques(gpu, sizes):
     check(gpu, sparse_with_cliques(30000, sizes, len(sizes)))
+
+
+# 5 M arcs: roots above 32 are scanned by a CTA each up to out-degree 64, and the graph with one of
+# 65 has a rank DAG
+@pytest.mark.parametrize("sizes", [(34, 50, 65), (66,)])
+def test_planted_cliques_in_a_large_graph(gpu, sizes):
+    check(gpu, sparse_with_cliques(850000, sizes, 7), p5=False)
 
 
 @pytest.mark.parametrize("n,ef,a,b", [(300, 3, .45, .1375), (2500, 16, .45, .1375),
