@@ -371,7 +371,8 @@ int jgpm_setop(int op, const int32_t* a, int32_t na, const int32_t* b, int32_t n
  * A = a[a_off[i] .. a_off[i+1]) and
  * B = b[b_off[i] .. b_off[i+1]), with per-pair bounds (upper/exclude arrays may be NULL).
  * Counts go to counts[i]; for the materialising ops results go to out[out_off[i] ..) where
- * out_off (nops+1 entries, host) gives each pair's capacity.  Host or device arrays. */
+ * out_off (nops+1 entries) gives each pair's capacity.  Host or device arrays.  A refused call
+ * (bad offsets, too little capacity) writes nothing. */
 int jgpm_setop_batch(int op, const int32_t* a, const int64_t* a_off, const int32_t* b,
                      const int64_t* b_off, int64_t nops, const int32_t* upper,
                      const int32_t* exclude, int32_t* counts, int32_t* out,

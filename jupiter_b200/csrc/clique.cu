@@ -27,8 +27,8 @@
 //                       lists in per-warp global scratch (the reference's scheme).
 // Measured (R-MAT scale 22, edge factor 4, per count): with level 1 as a scan of the rows
 // N+(v_i), searched in N+(u), the 4-clique count issued 5.9 G warp instructions and took
-// 6.5 ms, the 5-clique count 10.9 G and 14.7 ms; with the pair tests 1.65 G and 2.0 ms, 4.0 G
-// and 4.6 ms.
+// 6.5 ms, the 5-clique count 10.9 G and 14.7 ms; with the pair tests, by tiles, 1.24 G and
+// 1.5 ms, 2.86 G and 3.7 ms.
 //
 // Work is handed out by global atomic cursors (work stealing); roots are sorted by
 // descending out-degree so the heaviest start first.

@@ -128,7 +128,9 @@ __device__ __forceinline__ int32_t warp_owner(const int64_t* rowptr, int32_t n, 
 // the rows before each word, and the non-empty rows in order, so that an arc's owner is a popcount
 // and a load away and independent of the other arcs'.  (Walking the row ends from word to word
 // instead took three times as long on 33 M arcs: a chain of loads for every 32 arcs.)  On smaller
-// graphs (start == null), where its three launches cost more than they save, a search per word.
+// graphs (start == null), where its three launches cost more than they save, a search per word
+// (upload, checks, DAG and two counts of R-MAT graphs of edge factor 8, a = 0.45, by searches | bits:
+// 30,000 vertices, 0.4 M arcs: 470 | 492 us; 1,000,000, 16 M arcs: 2.66 | 2.57 ms; alike between).
 struct ArcOwners {
   const uint32_t* start = nullptr;
   const int32_t* before = nullptr;
