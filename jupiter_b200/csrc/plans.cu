@@ -174,8 +174,9 @@ struct PlanClique {
 
 // One root arc (v0, v1) of plan P, or the part of it that `split` names (plans of kSplitPlan; every
 // part builds the candidate list).  Returns the warp-uniform contribution; `lc` collects
-// per-lane partial contributions (summed at the end); `el` the set-op elements (lane 0).
-template <int P, bool STATS>
+// per-lane partial contributions (summed at the end); `el` the set-op elements (lane 0).  HUB: both
+// rows are long.
+template <int P, bool STATS, bool HUB = false>
 __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1, Lists& L,
                                           Split split, acc_t& lc, acc_t& el) {
   const int lane = threadIdx.x & 31;
@@ -217,7 +218,7 @@ __device__ __forceinline__ acc_t run_plan(const PlanArgs& a, vid_t v0, vid_t v1,
     int t = 0;
     if (P != kIC4 && P != kIPath4 && P != kIStar3) {
       if (STATS && lane == 0) el += (acc_t)d0 + d1;
-      t = warp_intersect(N0, d0, N1, d1, INT32_MAX, L.W);
+      t = warp_intersect<HUB>(N0, d0, N1, d1, INT32_MAX, L.W);
     }
     if (P == kP3) {
       // v2 in T = W above v1, v2 != v3: |N3| less v0 (always in N3), v1 and v2 where they are in it
@@ -561,7 +562,7 @@ __global__ void __launch_bounds__(256) k_plan_heavy(PlanArgs a) {
     t = __shfl_sync(kFull, t, 0);
     if ((int64_t)t >= arcs * kHeavyParts) break;
     const int2 arc = a.heavy[t / kHeavyParts];
-    uc += run_plan<P, false>(a, arc.x, arc.y, L, Split{(int)(t % kHeavyParts), kHeavyParts}, lc,
+    uc += run_plan<P, false, true>(a, arc.x, arc.y, L, Split{(int)(t % kHeavyParts), kHeavyParts}, lc,
                              el);
   }
   for (int o = 16; o > 0; o >>= 1) lc += __shfl_xor_sync(kFull, lc, o);

@@ -188,7 +188,9 @@ __device__ __forceinline__ int warp_intersect_count(const int32_t* a, int na, co
   return warp_sum_int(c);
 }
 
-// Materialises {x in A & B : x < upper} in ascending order into out; returns the size.
+// Materialises {x in A & B : x < upper} in ascending order into out; returns the size.  LONG: four
+// searches per lane at a time (warp_lookup), for lists of hundreds of ids.
+template <bool LONG = false>
 __device__ __forceinline__ int warp_intersect(const int32_t* a, int na, const int32_t* b,
                                               int nb, int32_t upper, int32_t* out) {
   const int lane = threadIdx.x & 31;
@@ -200,13 +202,20 @@ __device__ __forceinline__ int warp_intersect(const int32_t* a, int na, const in
     int tn = na; na = nb; nb = tn;
   }
   int written = 0;
-  for (int base = 0; base < na; base += 32) {
-    const int i = base + lane;
-    const int32_t key = i < na ? __ldg(a + i) : 0;
-    const bool f = i < na && contains_g(b, nb, key);
+  auto put = [&](int32_t key, bool valid, bool in_b) {
+    const bool f = valid && in_b;
     const unsigned mask = __ballot_sync(kFull, f);
     if (f) out[written + __popc(mask & ((1u << lane) - 1))] = key;
     written += __popc(mask);
+  };
+  if (LONG) {
+    warp_lookup(a, na, b, nb, put);
+  } else {
+    for (int base = 0; base < na; base += 32) {
+      const int i = base + lane;
+      const int32_t key = i < na ? __ldg(a + i) : 0;
+      put(key, i < na, i < na && contains_g(b, nb, key));
+    }
   }
   __syncwarp();
   return written;
